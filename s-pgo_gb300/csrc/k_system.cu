@@ -12,6 +12,7 @@
 // kept about a nearby camera centre, so the working precision (FP32 in the
 // mixed path) never sees world-sized lever arms.
 // g(i) = Ad_i^T sum_{lo <= i < hi} m_{lo,hi} is the e = 0 diagonal of the same sums.
+#include <algorithm>
 #include <type_traits>
 #include "kernels.cuh"
 #include "frames.cuh"
@@ -552,10 +553,125 @@ __global__ void __launch_bounds__(256) k_schur(PlanView pv, WorkView wv, Params 
   }
 }
 
+// ---- the FP64 path's Schur complement -------------------------------------------
+// Bound by the FP64 pipe (2 FMA per SM and cycle on this part: everything else in the
+// kernel is hidden behind it), so what counts is how many FP64 warp instructions it
+// issues.  A landmark's column of W is non-zero only in its own window [lo, hi) of pose
+// blocks, about 70 % of a circle problem's poses and 20 of a corridor's hundreds.  A warp
+// owns 2 x 4 pose blocks of the 48x48 tile (3x3 outputs a lane) and multiplies only the
+// landmarks whose window meets both its rows and its columns (one ballot per chunk); the
+// warps above the diagonal of a diagonal tile do nothing, and 1 / D is formed once per
+// landmark instead of once per tile row.  Counted on config-3 problems, this leaves 1.37x
+// the FMAs of the exact per-landmark lower triangles, against 4.6x for whole tiles (a
+// 1 x 8 block warp shape: 1.62x).  256-problem batch: 11.7 -> 4.1 ms a launch; one 10-pose
+// window, whose 6 items left the GPU empty, 235 -> about 90 us.
+// blockIdx.y splits an item's chunks where the plan has too few items to fill the GPU.
+__global__ void __launch_bounds__(256) k_schur_f64(PlanView pv, WorkView wv, Params prm, int gate) {
+  const int w = blockIdx.x;
+  const int b = pv.wk_prob[w];
+  if (!problem_active(wv.lm, b, gate)) return;
+  const int c0 = pv.wk_cbeg[w], len = pv.wk_cend[w] - c0;
+  const int kb = c0 + len * (int)blockIdx.y / (int)gridDim.y, ke = c0 + len * ((int)blockIdx.y + 1) / (int)gridDim.y;
+  if (kb >= ke) return;
+  const int ti = pv.wk_ti[w], tj = pv.wk_tj[w];
+  const int P = 6 * pv.p_npose[b];
+  const double lam1 = 1.0 + wv.lm[b].lam, eps = (double)prm.eps;
+  constexpr int TR = 6 * SPGO_TILE_BLOCKS;  // 48
+  __shared__ double WI[TR][SPGO_CHUNK + 1];
+  __shared__ double WJ[TR][SPGO_CHUNK + 1];  // scaled by 1 / D
+  __shared__ double dv[2][SPGO_CHUNK];
+  __shared__ double gs[2][SPGO_CHUNK];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool diag = ti == tj;
+  const int wr = warp >> 1, wc = warp & 1;
+  const int br = SPGO_TILE_BLOCKS * ti + 2 * wr, bc = SPGO_TILE_BLOCKS * tj + 4 * wc;  // the warp's first blocks
+  const bool idle = diag && 2 * wr + 1 < 4 * wc;                                        // above the diagonal
+  const int tr = 12 * wr + 3 * (lane >> 3), tc = 24 * wc + 3 * (lane & 7);              // the lane's first outputs
+  double acc[3][3];
+#pragma unroll
+  for (int x = 0; x < 3; ++x)
+#pragma unroll
+    for (int y = 0; y < 3; ++y) acc[x][y] = 0.0;
+  double accg = 0.0;
+  const double *Cv = reinterpret_cast<const double *>(wv.C);
+  const double *gav = reinterpret_cast<const double *>(wv.ga);
+  const double *slab_all = reinterpret_cast<const double *>(wv.slab);
+  auto scales = [&](int k) {  // lane = landmark of chunk k: 1 / D and g_a
+    const int c = pv.wk_chunks[k];
+    const int lm0 = pv.ch_lm0[c], cnt = pv.ch_cnt[c];
+    dv[k & 1][lane] = lane < cnt ? 1.0 / (Cv[lm0 + lane] * lam1 + eps) : 0.0;
+    gs[k & 1][lane] = lane < cnt ? gav[lm0 + lane] : 0.0;
+  };
+  if (warp == 0) scales(kb);
+  for (int k = kb; k < ke; ++k) {
+    const int c = pv.wk_chunks[k];
+    const int f0 = pv.ch_f0[c], nb = pv.ch_nb[c], lm0 = pv.ch_lm0[c], cnt = pv.ch_cnt[c];
+    const double *slab = slab_all + pv.ch_slab[c];
+    // this chunk's rows of the tile, before the barrier that ends the previous chunk
+    constexpr int RPW = TR / 8;
+    const int ri = 6 * (SPGO_TILE_BLOCKS * ti - f0) + warp, rj = 6 * (SPGO_TILE_BLOCKS * tj - f0) + warp;
+    double vi[RPW], vj[RPW];
+#pragma unroll
+    for (int q = 0; q < RPW; ++q) {
+      const int r = ri + 8 * q, s = rj + 8 * q;
+      vi[q] = r >= 0 && r < 6 * nb ? slab[(size_t)r * SPGO_CHUNK + lane] : 0.0;
+      vj[q] = diag ? vi[q] : (s >= 0 && s < 6 * nb ? slab[(size_t)s * SPGO_CHUNK + lane] : 0.0);
+    }
+    const int lo = lane < cnt ? pv.lm_lo[lm0 + lane] : 0, hi = lane < cnt ? pv.lm_hi[lm0 + lane] : 0;
+    __syncthreads();
+    const double d = dv[k & 1][lane];
+#pragma unroll
+    for (int q = 0; q < RPW; ++q) {
+      WI[warp + 8 * q][lane] = vi[q];
+      WJ[warp + 8 * q][lane] = vj[q] * d;
+    }
+    __syncthreads();
+    if (warp == 7 && k + 1 < ke) scales(k + 1);
+    // (a 1 / D that is not finite is never skipped: it has to reach S and fail the factor)
+    const bool bad = (((unsigned)__double2hiint(d) >> 20) & 0x7ffu) == 0x7ffu;
+    unsigned m = __ballot_sync(0xffffffffu, !idle && (bad || (lo < br + 2 && hi > br && lo < bc + 4 && hi > bc)));
+    while (m) {
+      const int kk = __ffs(m) - 1;
+      m &= m - 1;
+      const double a0 = WI[tr][kk], a1 = WI[tr + 1][kk], a2 = WI[tr + 2][kk];
+      const double b0 = WJ[tc][kk], b1 = WJ[tc + 1][kk], b2 = WJ[tc + 2][kk];
+      acc[0][0] += a0 * b0; acc[0][1] += a0 * b1; acc[0][2] += a0 * b2;
+      acc[1][0] += a1 * b0; acc[1][1] += a1 * b1; acc[1][2] += a1 * b2;
+      acc[2][0] += a2 * b0; acc[2][1] += a2 * b1; acc[2][2] += a2 * b2;
+    }
+    if (diag && tid < TR) {  // g_L row: the scaled rows times g_a
+      for (int kk = 0; kk < cnt; ++kk) accg += WJ[tid][kk] * gs[k & 1][kk];
+    }
+  }
+  double *SL = reinterpret_cast<double *>(wv.SL) + pv.p_S_off[b];
+#pragma unroll
+  for (int x = 0; x < 3; ++x) {
+    const int row = TR * ti + tr + x;
+#pragma unroll
+    for (int y = 0; y < 3; ++y) {
+      const int col = TR * tj + tc + y;
+      if (row < P && col <= row && acc[x][y] != 0.0) red_add(SL + (size_t)row * P + col, acc[x][y]);
+    }
+  }
+  if (diag && tid < TR) {
+    const int row = TR * ti + tid;
+    if (row < P && accg != 0.0) red_add(reinterpret_cast<double *>(wv.gL) + pv.p_param_off[b] + row, accg);
+  }
+}
+
+constexpr int kSmCount = 152;
+
 template <typename T>
 int launch_schur(const PlanView &pv, const WorkView &wv, const Params &prm, void *stream) {
   if (pv.n_items == 0) return 0;
-  k_schur<T><<<pv.n_items, 256, 0, (cudaStream_t)stream>>>(pv, wv, prm, GATE_RUNNING);
+  if constexpr (std::is_same<T, double>::value) {
+    // a chunk of one tile keeps an SM's FP64 pipe busy for several microseconds, so items
+    // are split down to single chunks until there are four CTAs per SM
+    const int sub = std::max(1, std::min(pv.wk_max_len, (4 * kSmCount + pv.n_items - 1) / pv.n_items));
+    k_schur_f64<<<dim3(pv.n_items, sub), 256, 0, (cudaStream_t)stream>>>(pv, wv, prm, GATE_RUNNING);
+  } else {
+    k_schur<T><<<pv.n_items, 256, 0, (cudaStream_t)stream>>>(pv, wv, prm, GATE_RUNNING);
+  }
   ++g_launches;
   return (int)cudaGetLastError();
 }
