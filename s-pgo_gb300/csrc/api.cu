@@ -880,7 +880,8 @@ static int enqueue_factor(spgo_solver *s, cudaStream_t st) {
     PROF(K_FACTOR);
     CUDA_TRY(launch_factor_solve<T>(s->pv, s->wv, s->prm, mixed, st));
     for (const int b : s->plan->large)
-      CUDA_TRY(launch_factor_large<T>(s->pv, s->wv, s->prm, b, 6 * s->plan->p_npose[b], s->plan->p_param_off[b],
+      CUDA_TRY(launch_factor_large<T>(s->pv, s->wv, s->prm, b, s->plan->p_npose[b], s->plan->p_pair_D[b],
+                                      s->plan->p_param_off[b],
                                       (mixed && !(s->prm.outer_steps > 0 && s->wv.facs)) ? s->prm.refine_steps : 0,
                                       st, s->side, s->ev_fork, s->ev_join));
   }
@@ -915,7 +916,8 @@ static int enqueue_candidate(spgo_solver *s, cudaStream_t st, bool solved = fals
     CUDA_TRY(launch_resid_solve(s->pv, s->wv, s->prm, k == 0, st));
     for (const int b : s->plan->large) {
       CUDA_TRY(launch_resid_reduce_large(s->pv, s->wv, b, s->plan->p_npose[b], st));
-      CUDA_TRY(launch_refine_large(s->pv, s->wv, s->prm, b, 6 * s->plan->p_npose[b], s->plan->p_param_off[b], st));
+      CUDA_TRY(launch_refine_large(s->pv, s->wv, s->prm, b, s->plan->p_npose[b], s->plan->p_pair_D[b],
+                                   s->plan->p_param_off[b], st));
     }
     if (k + 1 < outer) CUDA_TRY(launch_pair_twists(s->pv, s->wv, st));
   }

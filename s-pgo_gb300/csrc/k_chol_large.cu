@@ -1,6 +1,10 @@
 // Large reduced camera systems: problems whose packed factor does not fit in one
 // CTA's shared memory (P beyond ~300 in FP32; config 1's 600 and config 2's 3000).
 //
+// On the mixed path, problems whose windows give S a band of at most 16 SPGO_BAND_MAX_H
+// (windows of 45 poses) go to k_chol_band.cu instead; what is below serves the FP64 path and
+// the wider bands.
+//
 // Same mathematics as k_factor_solve (S = A + lam diag(A) - S_L, Cholesky, one
 // refinement step with an exact residual), spread over the GPU instead of one CTA:
 //   k_lg_assemble  row per CTA: the FP32/T copy of S into the factor storage
@@ -559,12 +563,18 @@ __global__ void __launch_bounds__(256) k_lg_bwd(PlanView pv, WorkView wv, int b,
   }
 }
 
-// a failed factorisation (or a timed-out substitution) leaves no step
-__global__ void k_lg_zero_failed(PlanView pv, WorkView wv, int b) {
+// a failed factorisation (or a timed-out substitution) leaves no step.  band: the banded
+// assembly cleared S_L inside the band only; what a non-finite 1 / D may have spread beyond
+// it (such an S always fails the factor) goes here.
+__global__ void k_lg_zero_failed(PlanView pv, WorkView wv, int b, int band) {
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   if (!wv.lm[b].fail) return;
   const int P = 6 * pv.p_npose[b], po = pv.p_param_off[b];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P; i += gridDim.x * blockDim.x) wv.delta[po + i] = 0.0;
+  if (!band) return;
+  float *SL = reinterpret_cast<float *>(wv.SL) + pv.p_S_off[b];
+  const size_t n = (size_t)P * P, step = (size_t)gridDim.x * blockDim.x;
+  for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += step) SL[k] = 0.f;
 }
 
 // residual y = g0 - S x from the exact S, warp per row
@@ -575,11 +585,12 @@ __global__ void __launch_bounds__(256) k_lg_resid(PlanView pv, WorkView wv, int 
   const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= P) return;
   const auto *Sx = reinterpret_cast<const typename ExactS<T>::type *>(wv.Sx) + pv.p_S_off[b] + (size_t)i * P;
+  const int bw = 6 * pv.p_pair_D[b] - 1, j0 = max(0, i - bw), j1 = min(P, i + bw + 1);  // S's band
   double r;
   if constexpr (std::is_same<T, float>::value) {
     const float *xs = wv.lg_xs + 2 * (size_t)po;
     df acc = df_make(0.f);
-    for (int j = lane; j < P; j += 32) {
+    for (int j = j0 + lane; j < j1; j += 32) {
       const float2 s = Sx[j];
       acc = acc + df{s.x, s.y} * df{xs[2 * j], xs[2 * j + 1]};
     }
@@ -591,16 +602,30 @@ __global__ void __launch_bounds__(256) k_lg_resid(PlanView pv, WorkView wv, int 
     r = (double)acc.h + (double)acc.l;
   } else {
     double acc = 0.0;
-    for (int j = lane; j < P; j += 32) acc += Sx[j] * wv.lg_x[po + j];
+    for (int j = j0 + lane; j < j1; j += 32) acc += Sx[j] * wv.lg_x[po + j];
     r = warp_sum(acc);
   }
   if (lane == 0) reinterpret_cast<T *>(wv.lg_y)[po + i] = (T)(wv.lg_g0[po + i] - r);
 }
 
 template <typename T>
-int launch_factor_large(const PlanView &pv, const WorkView &wv, const Params &prm, int b, int P, int param_off,
+int launch_factor_large(const PlanView &pv, const WorkView &wv, const Params &prm, int b, int N, int D, int param_off,
                         int refine, void *stream, void *side, void *ev_a, void *ev_b) {
   cudaStream_t st = (cudaStream_t)stream;
+  const int P = 6 * N;
+  if (std::is_same<T, float>::value && band_route(N, D)) {
+    int rc = launch_band_factor(pv, wv, prm, b, N, D, refine > 0, stream);
+    for (int it = 0; rc == 0 && it <= refine; ++it) {
+      if (it > 0) {
+        k_lg_resid<T><<<(P + 7) / 8, 256, 0, st>>>(pv, wv, b);
+        ++g_launches;
+      }
+      rc = launch_band_solve(pv, wv, prm, b, N, D, it == 0, it == refine, 0, stream);
+    }
+    k_lg_zero_failed<<<grid_for(P, 256), 256, 0, st>>>(pv, wv, b, 1);
+    ++g_launches;
+    return rc ? rc : (int)cudaGetLastError();
+  }
   const uint64_t wait_ns = wait_limit_ns(prm);
   k_lg_assemble<T><<<P, 256, 0, st>>>(pv, wv, b);
   int n = 1;
@@ -659,7 +684,7 @@ int launch_factor_large(const PlanView &pv, const WorkView &wv, const Params &pr
     k_lg_bwd<T><<<nblk, 256, 0, st>>>(pv, wv, b, it == 0, it == refine, 0, wait_ns);
     n += 2;
   }
-  k_lg_zero_failed<<<grid_for(P, 256), 256, 0, st>>>(pv, wv, b);
+  k_lg_zero_failed<<<grid_for(P, 256), 256, 0, st>>>(pv, wv, b, 0);
   ++n;
   g_launches += n;
   return (int)cudaGetLastError();
@@ -667,9 +692,11 @@ int launch_factor_large(const PlanView &pv, const WorkView &wv, const Params &pr
 
 // one refinement correction of the mixed path: the right-hand side is in lg_y
 // (k_resid_solve); delta += S^-1 lg_y with the factor of this iteration
-int launch_refine_large(const PlanView &pv, const WorkView &wv, const Params &prm, int b, int P, int param_off,
+int launch_refine_large(const PlanView &pv, const WorkView &wv, const Params &prm, int b, int N, int D, int param_off,
                         void *stream) {
+  if (band_route(N, D)) return launch_band_solve(pv, wv, prm, b, N, D, 0, 0, 1, stream);
   cudaStream_t st = (cudaStream_t)stream;
+  const int P = 6 * N;
   const uint64_t wait_ns = wait_limit_ns(prm);
   const int nblk = (P + kLgNB - 1) / kLgNB;
   int *ff = wv.lg_flag + param_off, *fb = wv.lg_flag + pv.total_params + param_off;
@@ -683,9 +710,9 @@ int launch_refine_large(const PlanView &pv, const WorkView &wv, const Params &pr
   return (int)cudaGetLastError();
 }
 
-template int launch_factor_large<float>(const PlanView &, const WorkView &, const Params &, int, int, int, int,
+template int launch_factor_large<float>(const PlanView &, const WorkView &, const Params &, int, int, int, int, int,
                                         void *, void *, void *, void *);
-template int launch_factor_large<double>(const PlanView &, const WorkView &, const Params &, int, int, int, int,
+template int launch_factor_large<double>(const PlanView &, const WorkView &, const Params &, int, int, int, int, int,
                                          void *, void *, void *, void *);
 
 }  // namespace spgo

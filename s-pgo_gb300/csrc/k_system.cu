@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(256) k_schur(PlanView pv, WorkView wv, Params 
 #pragma unroll
     for (int y = 0; y < 3; ++y) {
       const int col = TR * tj + 3 * tc + y;
-      if (col < P && acc[x][y] != T(0)) red_add(SL + (size_t)row * P + col, acc[x][y]);
+      if (col <= row && acc[x][y] != T(0)) red_add(SL + (size_t)row * P + col, acc[x][y]);  // (the lower triangle)
     }
   }
   if (diag && tid < TR) {

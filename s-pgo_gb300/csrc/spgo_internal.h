@@ -22,6 +22,7 @@
 #define SPGO_KSPLIT 16         // chunks per Schur work item
 #define SPGO_TC_SPLIT 64       // chunks per tensor-core Schur work item
 #define SPGO_FACTOR_SMEM (200 * 1024)  // shared-memory budget of the batched factorisation
+#define SPGO_BAND_MAX_H 17     // widest band of the banded factorisation, in 16-wide blocks
 
 namespace spgo {
 
@@ -172,8 +173,15 @@ template <typename T>
 int launch_schur(const PlanView &pv, const WorkView &wv, const Params &prm, void *stream);
 size_t factor_packed_bytes(int P, size_t ts);  // shared memory of the batched factorisation
 template <typename T>
-int launch_factor_large(const PlanView &pv, const WorkView &wv, const Params &prm, int b, int P, int param_off,
+int launch_factor_large(const PlanView &pv, const WorkView &wv, const Params &prm, int b, int N, int D, int param_off,
                         int refine, void *stream, void *side = nullptr, void *ev_a = nullptr, void *ev_b = nullptr);
+// banded factorisation and substitutions (k_chol_band.cu, mixed path): N poses, windows of
+// at most D of them
+bool band_route(int N, int D);
+int launch_band_factor(const PlanView &pv, const WorkView &wv, const Params &prm, int b, int N, int D, int sx,
+                       void *stream);
+int launch_band_solve(const PlanView &pv, const WorkView &wv, const Params &prm, int b, int N, int D, int first,
+                      int last, int accum, void *stream);
 template <typename T>
 int launch_factor_solve(const PlanView &pv, const WorkView &wv, const Params &prm, int mixed,
                         void *stream);
@@ -183,7 +191,7 @@ int launch_resid_pass(const PlanView &pv, const WorkView &wv, const Params &prm,
                       void *stream);
 int launch_resid_solve(const PlanView &pv, const WorkView &wv, const Params &prm, int first, void *stream);
 int launch_resid_reduce_large(const PlanView &pv, const WorkView &wv, int b, int N, void *stream);
-int launch_refine_large(const PlanView &pv, const WorkView &wv, const Params &prm, int b, int P, int param_off,
+int launch_refine_large(const PlanView &pv, const WorkView &wv, const Params &prm, int b, int N, int D, int param_off,
                         void *stream);
 int launch_backsub_refined(const PlanView &pv, const WorkView &wv, const Params &prm, const double *alpha,
                            double *alpha_out, void *stream);
