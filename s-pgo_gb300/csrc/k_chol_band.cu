@@ -163,11 +163,11 @@ __device__ __forceinline__ void bd_update(float *Cb, const float *Lr, const floa
 }
 
 // one warp: the 32x16 panel of a diagonal block B (Cholesky, lanes 0..15 = its rows) and the
-// block X below it (X L^-T, lanes 16..31; written back, and to gx, when `below`).  Four columns
-// at a time: every lane takes the 4x4 pivot block by shuffles and factors it redundantly, so
-// the serial chain per column is a reciprocal square root and a few FMAs with no shuffle in
-// it; the rows' entries and the rank-4 update (the other rows' entries through xs, 32 x 4)
-// follow.  Returns whether every pivot was positive.
+// block X below it (X L^-T, lanes 16..31, when `below`).  Four columns at a time: every lane
+// takes the 4x4 pivot block by shuffles and factors it redundantly, so the serial chain per
+// column is a reciprocal square root and a few FMAs with no shuffle in it; the rows' entries
+// and the rank-4 update (the other rows' entries through xs) follow.  Returns whether every
+// pivot was positive.
 __device__ __forceinline__ bool bd_panel(float *B, float *X, bool below, float *rinv_out, float *xs, int lane) {
   const int i = lane & 15;
   float *mine = (lane < kBb ? B : X) + i;

@@ -24,6 +24,7 @@
 #include "frames.cuh"
 #include "dfloat.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace spgo {
@@ -930,7 +931,7 @@ __device__ __forceinline__ void compose34_df(const df *A, const df *B, df *C) {
   }
 }
 
-// (also the FP64 copies, h + l, which the FP64 reduction of the pose-pair records reads)
+// (also the left centre as FP64, h + l, which the refinement's FP64 sums read)
 __device__ __forceinline__ void write_frame_df(const WorkView &wv, size_t f, const df *G, const df *Trl) {
   df Gr[12];
   compose34_df(G, Trl, Gr);
@@ -942,33 +943,58 @@ __device__ __forceinline__ void write_frame_df(const WorkView &wv, size_t f, con
       wv.fr_Rf[f * 18 + 9 + 3 * i + j] = Gr[4 * i + j].h;
       wv.fr_Rl[f * 18 + 3 * i + j] = G[4 * i + j].l;
       wv.fr_Rl[f * 18 + 9 + 3 * i + j] = Gr[4 * i + j].l;
-      wv.fr_Rd[f * 18 + 3 * i + j] = (double)G[4 * i + j].h + (double)G[4 * i + j].l;
-      wv.fr_Rd[f * 18 + 9 + 3 * i + j] = (double)Gr[4 * i + j].h + (double)Gr[4 * i + j].l;
     }
     wv.fr_ch[f * 6 + i] = G[4 * i + 3].h;
     wv.fr_ch[f * 6 + 3 + i] = Gr[4 * i + 3].h;
     wv.fr_cl[f * 6 + i] = G[4 * i + 3].l;
     wv.fr_cl[f * 6 + 3 + i] = Gr[4 * i + 3].l;
     wv.fr_c[f * 6 + i] = (double)G[4 * i + 3].h + (double)G[4 * i + 3].l;
-    wv.fr_c[f * 6 + 3 + i] = (double)Gr[4 * i + 3].h + (double)Gr[4 * i + 3].l;
   }
 }
 
-__global__ void k_chain_df(PlanView pv, WorkView wv, const double *__restrict__ poses, int gate) {
-  const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (b >= pv.B) return;
+// M_k <- M_0 M_1 ... M_k over the first n lanes of a warp (earlier factors on the left)
+__device__ __forceinline__ void scan34_df(df *M, int lane, int n) {
+#pragma unroll 1
+  for (int d = 1; d < n; d <<= 1) {
+    df P[12];
+#pragma unroll
+    for (int q = 0; q < 12; ++q)
+      P[q] = df{__shfl_up_sync(0xffffffffu, M[q].h, d), __shfl_up_sync(0xffffffffu, M[q].l, d)};
+    if (lane >= d) {
+      df C[12];
+      compose34_df(P, M, C);
+#pragma unroll
+      for (int q = 0; q < 12; ++q) M[q] = C[q];
+    }
+  }
+}
+
+// One CTA per problem, 32 frames a warp (one warp for the windows of a batch, up to
+// kChainWarps for a long trajectory): each warp scans its frames, warp 0 scans the warps'
+// totals onto the carry of the pass before.  The chain is latency: one warp walking 500
+// poses in 16 passes took 135 us, eight warps in two passes 36 us (one 20-pose window: 13.8 -> 9.0 us).
+constexpr int kChainWarps = 8;
+
+__global__ void __launch_bounds__(32 * kChainWarps) k_chain_df(PlanView pv, WorkView wv,
+                                                               const double *__restrict__ poses, int gate) {
+  __shared__ df tot[kChainWarps][12];   // a warp's product, then everything before it
+  __shared__ df carry_s[12];
+  const int b = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   if (!problem_active(wv.lm, b, gate)) return;
   const int N = pv.p_npose[b], fo = pv.p_frame_off[b], po = pv.p_pose_off[b];
   df Trl[12], carry[12];
+  {
+    const df t = df_from_double(pv.p_Trl[12 * b + min(lane, 11)]);  // lane q converts entry q for the warp
 #pragma unroll
-  for (int q = 0; q < 12; ++q) {
-    Trl[q] = df_from_double(pv.p_Trl[12 * b + q]);
-    carry[q] = df_make((q == 0 || q == 5 || q == 10) ? 1.f : 0.f);
+    for (int q = 0; q < 12; ++q) {
+      Trl[q] = df{__shfl_sync(0xffffffffu, t.h, q), __shfl_sync(0xffffffffu, t.l, q)};
+      carry[q] = df_make((q == 0 || q == 5 || q == 10) ? 1.f : 0.f);
+    }
   }
-  if (lane == 0) write_frame_df(wv, (size_t)fo, carry, Trl);
-  for (int s = 0; s < N; s += 32) {
-    const int k = s + lane;
+  if (threadIdx.x == 0) write_frame_df(wv, (size_t)fo, carry, Trl);
+  for (int s = 0; s < N; s += 32 * nw) {
+    const int k = s + threadIdx.x;
     df M[12];
 #pragma unroll
     for (int q = 0; q < 12; ++q) M[q] = df_make((q == 0 || q == 5 || q == 10) ? 1.f : 0.f);
@@ -985,25 +1011,46 @@ __global__ void k_chain_df(PlanView pv, WorkView wv, const double *__restrict__ 
                                 Td[11]);
       }
     }
-    // inclusive scan: M_k <- M_0 M_1 ... M_k (earlier factors on the left)
+    scan34_df(M, lane, min(32, N - s));
+    if (nw > 1) {
+      if (lane == 31) {
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      df P[12];
-#pragma unroll
-      for (int q = 0; q < 12; ++q)
-        P[q] = df{__shfl_up_sync(0xffffffffu, M[q].h, d), __shfl_up_sync(0xffffffffu, M[q].l, d)};
-      if (lane >= d) {
-        df C[12];
-        compose34_df(P, M, C);
-#pragma unroll
-        for (int q = 0; q < 12; ++q) M[q] = C[q];
+        for (int q = 0; q < 12; ++q) tot[warp][q] = M[q];
       }
-    }
-    df G[12];
-    compose34_df(carry, M, G);
-    if (k < N) write_frame_df(wv, (size_t)(fo + k + 1), G, Trl);
+      __syncthreads();
+      if (warp == 0) {  // lane w < nw: the carry and the products of the warps before w; lane nw: the next carry
+        df E[12];
 #pragma unroll
-    for (int q = 0; q < 12; ++q) carry[q] = df{__shfl_sync(0xffffffffu, G[q].h, 31), __shfl_sync(0xffffffffu, G[q].l, 31)};
+        for (int q = 0; q < 12; ++q) E[q] = lane == 0 || lane > nw ? carry[q] : tot[lane - 1][q];
+        scan34_df(E, lane, nw + 1);
+        __syncwarp();
+        if (lane < nw) {
+#pragma unroll
+          for (int q = 0; q < 12; ++q) tot[lane][q] = E[q];
+        } else if (lane == nw) {
+#pragma unroll
+          for (int q = 0; q < 12; ++q) carry_s[q] = E[q];
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < 12; ++q) carry[q] = tot[warp][q];
+    }
+    if (k < N) {
+      df G[12];
+      compose34_df(carry, M, G);
+      write_frame_df(wv, (size_t)(fo + k + 1), G, Trl);
+    }
+    if (nw > 1) {
+#pragma unroll
+      for (int q = 0; q < 12; ++q) carry[q] = carry_s[q];
+      __syncthreads();  // (the next pass writes tot and carry_s)
+    } else if (s + 32 < N) {
+      df G[12];
+      compose34_df(carry, M, G);
+#pragma unroll
+      for (int q = 0; q < 12; ++q) carry[q] = df{__shfl_sync(0xffffffffu, G[q].h, 31), __shfl_sync(0xffffffffu, G[q].l, 31)};
+    }
   }
 }
 
@@ -1011,7 +1058,8 @@ int launch_chain(const PlanView &pv, const WorkView &wv, const double *poses, in
   if (f64)
     k_chain<<<pv.B, 32, 0, (cudaStream_t)stream>>>(pv, wv, poses, gate);  // one warp (and SM slot) per problem
   else
-    k_chain_df<<<pv.B, 32, 0, (cudaStream_t)stream>>>(pv, wv, poses, gate);
+    k_chain_df<<<pv.B, 32 * std::min(kChainWarps, std::max(1, (pv.max_P / 6 + 31) / 32)), 0, (cudaStream_t)stream>>>(
+        pv, wv, poses, gate);
   ++g_launches;
   return (int)cudaGetLastError();
 }

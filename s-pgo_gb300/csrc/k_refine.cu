@@ -36,6 +36,8 @@
 //
 // Replaces nothing in the reference, whose GPU step is an FP32 Gauss-Newton step
 // solved once (src/Optimization/Solver_cuda.cu:594-782, linear_solvers.cu:195-218).
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "frames.cuh"
 #include "dfloat.cuh"
@@ -58,7 +60,7 @@ __device__ __forceinline__ void frame_Rc(const WorkView &wv, int f, double *R, d
 #pragma unroll
   for (int k = 0; k < 9; ++k) R[k] = (double)Rh[k] + (double)Rl[k];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) c[k] = (double)wv.fr_ch[(size_t)f * 6 + k] + (double)wv.fr_cl[(size_t)f * 6 + k];
+  for (int k = 0; k < 3; ++k) c[k] = wv.fr_c[(size_t)f * 6 + k];
 }
 
 // a problem takes (the next step of) the refinement: running, its step not failed, and
@@ -72,22 +74,30 @@ __device__ __forceinline__ bool refine_active(const WorkView &wv, int b) {
 // convention of the pose blocks, k_system.cu).  With the prefix sums
 // Om(k) = sum_{i<k} R_i psi_i and V(k) = sum_{i<k} c_i x R_i psi_i + R_i rho_i,
 // W(lo, hi) = [Om(hi) - Om(lo) ; V(hi) - V(lo) - c_lo x (Om(hi) - Om(lo))].
+// Only differences of the prefix sums enter, so a CTA takes kTwSlice consecutive lo's and
+// sums over their own poses and the D after them: a batch's windows are one CTA each, a long
+// trajectory spreads over the GPU (500 poses: 141 us on one SM's FP64 pipe, 12 us spread out).
 constexpr int kTwThreads = 128;
+constexpr int kTwSlice = 32;
 
 __global__ void __launch_bounds__(kTwThreads) k_pair_twists(PlanView pv, WorkView wv) {
-  extern __shared__ double tw_s[];  // [(N + 1) * 6]
-  const int b = blockIdx.x;
-  if (!refine_active(wv, b)) return;
+  __shared__ double tw_s[(kTwSlice + SPGO_MAX_WINDOW + 1) * 6];
+  const int b = blockIdx.x, l0 = kTwSlice * blockIdx.y;
   const int N = pv.p_npose[b], D = pv.p_pair_D[b], fo = pv.p_frame_off[b], po = pv.p_param_off[b];
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
-    double R[9], c[3];
-    frame_Rc(wv, fo + i, R, c);
-    const double *x = wv.delta + po + 6 * i;
+  if (l0 >= N || !refine_active(wv, b)) return;
+  const int n = min(N - l0, kTwSlice + D);  // the slice's poses and the D after them
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const float *Rh = wv.fr_Rf + (size_t)(fo + l0 + i) * 18, *Rl = wv.fr_Rl + (size_t)(fo + l0 + i) * 18;
+    const double *c = wv.fr_c + (size_t)(fo + l0 + i) * 6;
+    const double *x = wv.delta + po + 6 * (l0 + i);
     double w[3], v[3];
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
-      w[r] = R[3 * r] * x[0] + R[3 * r + 1] * x[1] + R[3 * r + 2] * x[2];
-      v[r] = R[3 * r] * x[3] + R[3 * r + 1] * x[4] + R[3 * r + 2] * x[5];
+      double R[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) R[k] = (double)Rh[3 * r + k] + (double)Rl[3 * r + k];
+      w[r] = R[0] * x[0] + R[1] * x[1] + R[2] * x[2];
+      v[r] = R[0] * x[3] + R[1] * x[4] + R[2] * x[5];
     }
     double *o = tw_s + (size_t)(i + 1) * 6;
     o[0] = w[0];
@@ -99,20 +109,27 @@ __global__ void __launch_bounds__(kTwThreads) k_pair_twists(PlanView pv, WorkVie
   }
   if (threadIdx.x < 6) tw_s[threadIdx.x] = 0.0;
   __syncthreads();
-  if (threadIdx.x < 6) {
-    double acc = 0.0;
-    for (int i = 1; i <= N; ++i) {
-      acc += tw_s[i * 6 + threadIdx.x];
-      tw_s[i * 6 + threadIdx.x] = acc;
+  for (int k = threadIdx.x >> 5; k < 6; k += kTwThreads / 32) {  // warp scan per component
+    const int lane = threadIdx.x & 31;
+    double carry = 0.0;
+    for (int s = 0; s < n; s += 32) {
+      double v = s + lane < n ? tw_s[(s + lane + 1) * 6 + k] : 0.0;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const double u = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += u;
+      }
+      v += carry;
+      if (s + lane < n) tw_s[(s + lane + 1) * 6 + k] = v;
+      carry = __shfl_sync(0xffffffffu, v, 31);
     }
   }
   __syncthreads();
-  float *out = wv.twist + (size_t)pv.p_pair_off[b] * 6;
-  for (int t = threadIdx.x; t < N * D; t += blockDim.x) {
-    const int lo = t / D, hi = lo + t % D + 1;
-    if (hi > N) continue;
-    double R[9], c[3];
-    frame_Rc(wv, fo + lo, R, c);
+  float *out = wv.twist + ((size_t)pv.p_pair_off[b] + (size_t)l0 * D) * 6;
+  for (int t = threadIdx.x; t < min(kTwSlice, N - l0) * D; t += blockDim.x) {
+    const int lo = t / D, hi = lo + t % D + 1;  // relative to l0
+    if (l0 + hi > N) continue;
+    const double *c = wv.fr_c + (size_t)(fo + l0 + lo) * 6;
     double dw[3], dv[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -130,8 +147,8 @@ __global__ void __launch_bounds__(kTwThreads) k_pair_twists(PlanView pv, WorkVie
 }
 
 int launch_pair_twists(const PlanView &pv, const WorkView &wv, void *stream) {
-  const size_t sm = (size_t)(pv.max_P / 6 + 1) * 6 * sizeof(double);
-  k_pair_twists<<<pv.B, kTwThreads, sm, (cudaStream_t)stream>>>(pv, wv);
+  const int slices = (pv.max_P / 6 + kTwSlice - 1) / kTwSlice;
+  k_pair_twists<<<dim3(pv.B, slices), kTwThreads, 0, (cudaStream_t)stream>>>(pv, wv);
   ++g_launches;
   return (int)cudaGetLastError();
 }
@@ -541,7 +558,7 @@ __global__ void __launch_bounds__(kRsThreads) k_resid_solve(PlanView pv, WorkVie
   double *rowm = cs + (size_t)(N + 1) * 3;            // [N + 1][6]: sum over hi of m(lo, hi)
   double *colm = rowm + (size_t)(N + 1) * 6;          // [N + 1][6]: sum over lo of n(lo, hi)
   for (int k = tid; k < N * 3; k += nt)
-    cs[k] = (double)wv.fr_ch[(size_t)(fo + k / 3) * 6 + k % 3] + (double)wv.fr_cl[(size_t)(fo + k / 3) * 6 + k % 3];
+    cs[k] = wv.fr_c[(size_t)(fo + k / 3) * 6 + k % 3];
   __syncthreads();
   double *recs = wv.pdual + (size_t)pv.p_pair_off[b] * 6;
   for (int t = tid; t < 12 * N; t += nt) {
@@ -652,16 +669,15 @@ __global__ void __launch_bounds__(kRsThreads) k_resid_solve(PlanView pv, WorkVie
 //                     into lg_y for the multi-CTA substitutions; clears the pair duals
 // The per-pose values are those of k_resid_solve; only the prefix is summed in another
 // order (FP64, segments of ~N / 42 poses).
-__global__ void __launch_bounds__(256) k_rs_sums_large(PlanView pv, WorkView wv, int b) {
+// (FP64-bound: small CTAs spread the sums over the SMs, and the centres come as FP64)
+__global__ void __launch_bounds__(64) k_rs_sums_large(PlanView pv, WorkView wv, int b) {
   if (!refine_active(wv, b)) return;
   const int N = pv.p_npose[b], D = pv.p_pair_D[b], fo = pv.p_frame_off[b];
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 12 * N) return;
   double *rowm = wv.lg_red + ((size_t)pv.p_pose_off[b] + b) * 12, *colm = rowm + (size_t)(N + 1) * 6;
   const double *recs = wv.pdual + (size_t)pv.p_pair_off[b] * 6;
-  auto cen = [&](int f, int k) {
-    return (double)wv.fr_ch[(size_t)(fo + f) * 6 + k] + (double)wv.fr_cl[(size_t)(fo + f) * 6 + k];
-  };
+  auto cen = [&](int f, int k) { return wv.fr_c[(size_t)(fo + f) * 6 + k]; };
   const int k = t % 6;
   if (t < 6 * N) {  // row lo = t / 6
     const int lo = t / 6;
@@ -708,8 +724,7 @@ __global__ void __launch_bounds__(256) k_rs_scan_large(PlanView pv, WorkView wv,
     const double *m = rowm + i * 6;
     double nrow = m[k];
     if (k < 3) {
-      const double c1 = (double)wv.fr_ch[(size_t)(fo + i) * 6 + k1] + (double)wv.fr_cl[(size_t)(fo + i) * 6 + k1];
-      const double c2 = (double)wv.fr_ch[(size_t)(fo + i) * 6 + k2] + (double)wv.fr_cl[(size_t)(fo + i) * 6 + k2];
+      const double c1 = wv.fr_c[(size_t)(fo + i) * 6 + k1], c2 = wv.fr_c[(size_t)(fo + i) * 6 + k2];
       nrow += c1 * m[3 + k2] - c2 * m[3 + k1];
     }
     val[t] = nrow - colm[t];
@@ -741,7 +756,7 @@ __global__ void __launch_bounds__(256) k_rs_scan_large(PlanView pv, WorkView wv,
   }
 }
 
-__global__ void __launch_bounds__(128) k_rs_rhs_large(PlanView pv, WorkView wv, int b) {
+__global__ void __launch_bounds__(64) k_rs_rhs_large(PlanView pv, WorkView wv, int b) {
   if (!refine_active(wv, b)) return;
   const int N = pv.p_npose[b], D = pv.p_pair_D[b], P = 6 * N;
   const int fo = pv.p_frame_off[b], po = pv.p_param_off[b];
@@ -778,11 +793,11 @@ __global__ void __launch_bounds__(128) k_rs_rhs_large(PlanView pv, WorkView wv, 
 int launch_resid_reduce_large(const PlanView &pv, const WorkView &wv, int b, int N, void *stream) {
   if (!wv.lg_red) return 0;  // (the FP64 path has no refinement)
   cudaStream_t st = (cudaStream_t)stream;
-  k_rs_sums_large<<<(12 * N + 255) / 256, 256, 0, st>>>(pv, wv, b);
+  k_rs_sums_large<<<(12 * N + 63) / 64, 64, 0, st>>>(pv, wv, b);
   const size_t sm = (size_t)N * 6 * sizeof(double);
   cudaFuncSetAttribute(k_rs_scan_large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   k_rs_scan_large<<<1, 256, sm, st>>>(pv, wv, b);
-  k_rs_rhs_large<<<(N + 127) / 128, 128, 0, st>>>(pv, wv, b);
+  k_rs_rhs_large<<<std::max((N + 63) / 64, 96), 64, 0, st>>>(pv, wv, b);  // (the clearing wants the CTAs)
   g_launches += 3;
   return (int)cudaGetLastError();
 }

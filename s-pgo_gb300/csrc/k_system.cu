@@ -313,18 +313,23 @@ __global__ void __launch_bounds__(128) k_pair_shift_df(PlanView pv, WorkView wv)
   for (int k = 0; k < 27; ++k) out[k] = v[k];
 }
 
-// one CTA per problem: 1. thread per (hi, component): prefix over lo,
-// P(i, hi) = sum_{lo <= i} M(lo, hi);  2. thread per (i, component): suffix over hi,
-// F(i, i + e) = sum_{d > e} P(i, i + d)
+// 1. thread per (hi, component): prefix over lo, P(i, hi) = sum_{lo <= i} M(lo, hi);
+// 2. thread per (i, component): suffix over hi, F(i, i + e) = sum_{d > e} P(i, i + d).
+// PHASE 0: both, one CTA per problem (the windows of a batch); 1, 2: one of them over a grid,
+// for trajectories of more than kPrWide poses (500 poses on one SM took 150 us, spread out
+// 12 us; at 32 poses one CTA's barrier is cheaper than a second launch).
+constexpr int kPrWide = 48;
+
+template <int PHASE>
 __global__ void __launch_bounds__(kPrThreads) k_pair_scan_df(PlanView pv, WorkView wv) {
   const int b = blockIdx.x;
   if (!problem_active(wv.lm, b, GATE_RELIN)) return;
   const int N = pv.p_npose[b], D = pv.p_pair_D[b];
-  const int tid = threadIdx.x, nt = blockDim.x;
+  const int tid = blockIdx.y * blockDim.x + threadIdx.x, nt = gridDim.y * blockDim.x;
   df *F = reinterpret_cast<df *>(wv.pairF) + (size_t)pv.p_pair_off[b] * 27;
   // the running sums: eight records loaded before any is summed and stored back (the
   // stores could alias later loads, so without that each step is a round trip)
-  for (int t = tid; t < N * 27; t += nt) {
+  for (int t = PHASE == 2 ? N * 27 : tid; t < N * 27; t += nt) {
     const int hi = t / 27 + 1, comp = t % 27;
     df s = df_make(0.f);
     for (int lo0 = max(0, hi - D); lo0 < hi; lo0 += 8) {
@@ -340,7 +345,8 @@ __global__ void __launch_bounds__(kPrThreads) k_pair_scan_df(PlanView pv, WorkVi
         }
     }
   }
-  __syncthreads();
+  if (PHASE == 1) return;
+  if (PHASE == 0) __syncthreads();
   for (int t = tid; t < N * 27; t += nt) {
     const int i = t / 27, comp = t % 27;
     df *base = F + (size_t)i * D * 27 + comp;
@@ -463,7 +469,14 @@ int launch_system(const PlanView &pv, const WorkView &wv, int gate, void *stream
   const int nd = pv.max_D > 0 ? pv.max_D : 1;
   if constexpr (std::is_same<T, float>::value) {
     k_pair_shift_df<<<dim3(grid_for((long long)nmax * nd, 128), pv.B), 128, 0, st>>>(pv, wv);
-    k_pair_scan_df<<<pv.B, kPrThreads, 0, st>>>(pv, wv);
+    if (nmax <= kPrWide) {
+      k_pair_scan_df<0><<<pv.B, kPrThreads, 0, st>>>(pv, wv);
+    } else {
+      const dim3 grid(pv.B, grid_for((long long)nmax * 27, 128));
+      k_pair_scan_df<1><<<grid, 128, 0, st>>>(pv, wv);
+      k_pair_scan_df<2><<<grid, 128, 0, st>>>(pv, wv);
+      ++g_launches;
+    }
     k_pairs_to_A_df<<<dim3(grid_for((long long)nmax * nd, 128), pv.B), 128, 0, st>>>(pv, wv);
     g_launches += 3;
   } else {

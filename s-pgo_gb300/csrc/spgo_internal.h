@@ -92,8 +92,8 @@ struct WorkView {
   // frame tables: [F][2 cams] rotation (cam->world) and centre
   float *fr_Rf;     // [F][2][9]
   float *fr_Rl;     // [F][2][9] float(R - float(R))
-  double *fr_Rd;    // [F][2][9]
-  double *fr_c;     // [F][2][3]
+  double *fr_Rd;    // [F][2][9] (FP64 path)
+  double *fr_c;     // [F][2][3] (mixed path: the left camera's)
   float *fr_ch;     // [F][2][3] float(c)
   float *fr_cl;     // [F][2][3] float(c - float(c))
   double *poses_cand;   // [NP][12]
