@@ -768,6 +768,7 @@ static void make_views(spgo_solver *s) {
   v.tc_chunks = seg_ptr<int32_t>(p, st, i++);
   v.fs_prob = seg_ptr<int32_t>(p, st, i++);
   v.n_tc_items = (int32_t)p->tc_prob.size();
+  v.n_tc_chunks = (int32_t)p->tc_chunks.size();
   for (size_t k = 0; k < p->wk_prob.size(); ++k) v.wk_max_len = std::max(v.wk_max_len, p->wk_cend[k] - p->wk_cbeg[k]);
   for (size_t k = 0; k < p->tc_prob.size(); ++k) v.tc_max_len = std::max(v.tc_max_len, p->tc_cend[k] - p->tc_cbeg[k]);
   v.max_P_small = p->max_P_small;

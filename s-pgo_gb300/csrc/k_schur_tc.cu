@@ -35,6 +35,8 @@
 // failure flag, lets the copies and MMAs in flight finish, frees TMEM and returns.
 //
 // (The SIMT Schur path in k_system.cu forms g_L the same way inside its tiles.)
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "tc.cuh"
 
@@ -116,7 +118,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_schur_tc(PlanView pv, WorkVie
   const int row0 = pv.tc_row0[w], col0 = pv.tc_col0[w], ncols = pv.tc_ncols[w];
   const bool diag = row0 == col0;
   const int P = 6 * pv.p_npose[b];
-  const int cb = pv.tc_cbeg[w], n = min(pv.tc_cend[w] - cb, kTcMaxChunks);
+  // blockIdx.y: this CTA's share of the item's chunks
+  const int len = pv.tc_cend[w] - pv.tc_cbeg[w], y = (int)blockIdx.y, ny = (int)gridDim.y;
+  const int cb = pv.tc_cbeg[w] + len * y / ny, n = min(pv.tc_cbeg[w] + len * (y + 1) / ny - cb, kTcMaxChunks);
+  if (n <= 0) return;
   const int ngroups = (n + kGroup - 1) / kGroup;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile int *err = &sm.err;
@@ -330,12 +335,36 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_schur_tc(PlanView pv, WorkVie
 
 size_t tc_smem_bytes() { return sizeof(TcSmem) + 1024; }
 
+// CTAs per work item.  A CTA spends about 13 chunks' time (0.85 us each) on starting (TMEM,
+// barriers) and on adding its tile into S_L, and an SM runs one at a time.  So with `sub`
+// CTAs per item a pass takes as long as all the work over the SMs, or as the longest share,
+// and half a CTA more where a second wave starts; the estimate is within 10 % of what was
+// measured (698 items of a 256-window batch: whole items, 246 us; the one 61-chunk item of a
+// 20-pose window, a chunk per CTA: 66 -> 14 us; 100 items of 35 chunks: two shares each took
+// 52 us, whole ones 44).
+static int tc_shares(const PlanView &pv) {
+  constexpr float kFixed = 13.f, kSms = 152.f;
+  const float n = (float)pv.n_tc_items, mean = (float)pv.n_tc_chunks / n;
+  int best = 1;
+  float t_best = 1e30f;
+  for (int sub = 1; sub <= std::max(1, pv.tc_max_len); ++sub) {
+    const float f = (float)sub, all = n * (mean + kFixed * f) / kSms;
+    float t = std::max(all, kFixed + (float)((pv.tc_max_len + sub - 1) / sub));
+    if (n * f > kSms) t += 0.5f * (kFixed + mean / f);
+    if (t < t_best) {
+      t_best = t;
+      best = sub;
+    }
+  }
+  return best;
+}
+
 int launch_schur_tc(const PlanView &pv, const WorkView &wv, const Params &prm, void *stream) {
   cudaStream_t st = (cudaStream_t)stream;
   if (pv.n_tc_items > 0) {
     const size_t sm = tc_smem_bytes();
     cudaFuncSetAttribute(k_schur_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_schur_tc<<<pv.n_tc_items, kTcThreads, sm, st>>>(pv, wv, prm, GATE_RUNNING);
+    k_schur_tc<<<dim3(pv.n_tc_items, tc_shares(pv)), kTcThreads, sm, st>>>(pv, wv, prm, GATE_RUNNING);
     ++g_launches;
   }
   return (int)cudaGetLastError();
