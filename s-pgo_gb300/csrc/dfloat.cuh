@@ -8,14 +8,17 @@
 // level the stopping rule needs.  FP64 would fix that but runs far slower than
 // FP32 on this part; double-float runs on the FP32 pipes.
 //
-// Requires IEEE float semantics (no fast-math reassociation); FMA contraction is
-// harmless here because the products that must be exact use fmaf explicitly.
+// Requires IEEE float semantics (no fast-math reassociation), and a product whose error
+// term is kept must not be contracted into a sum: a two-sum of fma(a, b, y) instead of
+// p + y, p = fl(a b), has p's error in its result already, and where p and y cancel the
+// two-sum's own error term does not take it out again, so that it counts twice (an error
+// of 2^-24 of p).  Hence the explicit rounding in two_prod.
 #pragma once
 #include <cuda_runtime.h>
 
 namespace spgo {
 
-struct df {
+struct __align__(8) df {  // (one 8-byte access)
   float h, l;
 };
 
@@ -38,7 +41,7 @@ __device__ __forceinline__ df fast_two_sum(float a, float b) {  // |a| >= |b|
 }
 
 __device__ __forceinline__ df two_prod(float a, float b) {
-  const float p = a * b;
+  const float p = __fmul_rn(a, b);  // (never contracted into a later addition, see above)
   return df{p, fmaf(a, b, -p)};
 }
 

@@ -12,8 +12,8 @@
 // So the FP32 system only preconditions.  Each refinement step forms the
 // residual of the whole damped system
 //   r_p = J_p^T W (r - J x) - lam diag(A) x_p,   r_a = J_a^T W (r - J x) - (lam C + eps) x_a
-// from the FP32 Jacobian, recomputed per observation, with every product J e
-// exact (two-product) and every sum in double-float / FP64, then applies the FP32
+// from the FP32 Jacobian rows, recomputed per observation as the linearisation formed
+// them (jac_rows.cuh), with every product J e exact (two-product) and every sum in double-float / FP64, then applies the FP32
 // system's inverse: x_p += S^-1 (r_p - W D^-1 r_a), x_a += D^-1 (r_a - W^T dx_p).
 // The first residual pass also sums the accurate gradient J^T W r, which the
 // predicted decrease of the gain ratio uses.
@@ -40,18 +40,10 @@
 
 #include "kernels.cuh"
 #include "frames.cuh"
-#include "dfloat.cuh"
+#include "jac_rows.cuh"
 #include "chol_subst.cuh"
 
 namespace spgo {
-
-// a b + c d exactly rounded to a double-float
-__device__ __forceinline__ df prod2(float a, float b, float c, float d) {
-  const df p = two_prod(a, b), q = two_prod(c, d);
-  df s = two_sum(p.h, q.h);
-  s.l += p.l + q.l;
-  return fast_two_sum(s.h, s.l);
-}
 
 // left camera of frame f: rotation (cam -> world) and centre, FP64 from the
 // double-float frame tables of the mixed path
@@ -170,24 +162,23 @@ struct RefSmem {
   float bt[2][SPGO_CHUNK];  // warps 0 and 1: partial W^T x_p over their slab row blocks
 };
 
-// dynamic shared memory (W = window frames): the window's rotations [W][18] (both
-// cameras) | the pair origins' offsets [W][4] | the pair twists [W][6] | the per-warp
-// staging [warps][2 x 6][33] float of the pair duals
+// dynamic shared memory (W = window frames): the pair origins' offsets [W][3] and the per-warp
+// staging [warps][6][33] of the pair duals (double-float) | the window's rotations [W][18]
+// (both cameras) | the pair twists [W][6]
 struct RpLayout {
-  size_t rw, xpo, tws, stage, total;
+  size_t xpo, stage, rw, tws, total;
   __host__ __device__ explicit RpLayout(int max_nb) {
     const size_t W = (size_t)max_nb + 1;
-    auto up = [](size_t x) { return (x + 15) & ~(size_t)15; };
-    rw = 0;
-    xpo = rw + up(W * 18 * sizeof(float));
-    tws = xpo + up(W * 4 * sizeof(float));
-    stage = tws + up(W * 6 * sizeof(float));
-    total = stage + (size_t)kRpWarps * 2 * 6 * kRpPitch * sizeof(float);
+    xpo = 0;
+    stage = xpo + W * 3 * sizeof(df);
+    rw = stage + (size_t)kRpWarps * 6 * kRpPitch * sizeof(df);
+    tws = rw + W * 18 * sizeof(float);
+    total = tws + W * 6 * sizeof(float);
   }
 };
 
 // The accurate gradient itself (J^T W r, pose and inverse-depth parts) comes from the
-// linearisation, which sums it exactly (k_linearize.cu, k_system.cu); each pass here
+// linearisation, which sums it exactly (k_jacobian.cu, k_system.cu); each pass here
 // forms only the duals of e.
 template <bool FIRST>
 __global__ void __launch_bounds__(kRpThreads, 8) k_resid_pass(PlanView pv, WorkView wv, Params prm,
@@ -218,9 +209,9 @@ __global__ void __launch_bounds__(kRpThreads, 8) k_resid_pass(PlanView pv, WorkV
   }
   const RpLayout lay(pv.max_nb);
   float *Rw = reinterpret_cast<float *>(smem_raw + lay.rw);
-  float *xpo = reinterpret_cast<float *>(smem_raw + lay.xpo);
+  df *xpo = reinterpret_cast<df *>(smem_raw + lay.xpo);
   float *tws = reinterpret_cast<float *>(smem_raw + lay.tws);
-  float *stage = reinterpret_cast<float *>(smem_raw + lay.stage);
+  df *stage = reinterpret_cast<df *>(smem_raw + lay.stage);
   const int D = pv.p_pair_D[b];
   const float *slab = reinterpret_cast<const float *>(wv.slab) + pv.ch_slab[c];
   const float *Cv = reinterpret_cast<const float *>(wv.C);
@@ -288,11 +279,15 @@ __global__ void __launch_bounds__(kRpThreads, 8) k_resid_pass(PlanView pv, WorkV
       Rw[idx] = wv.fr_Rf[(size_t)(fo + f0) * 18 + idx];
     for (int f = tid - 64; f < nb + 1; f += blockDim.x - 64) {
       const int n = f0 + f;
-      Vec3<float> d = v3<float>(0.f, 0.f, 0.f);
-      if (n < ah) d = FramesT<float>::rel(wv, fh, 0, fo + n, 0);
-      xpo[4 * f] = d.x;
-      xpo[4 * f + 1] = d.y;
-      xpo[4 * f + 2] = d.z;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        df d = df_make(0.f);
+        if (n < ah) {
+          const size_t x = (size_t)fh * 6 + k, y = (size_t)(fo + n) * 6 + k;
+          d = df_sub(wv.fr_ch[x], wv.fr_ch[y]) + df_make(wv.fr_cl[x] - wv.fr_cl[y]);
+        }
+        xpo[3 * f + k] = d;
+      }
       const int lo = min(ah, n), hi = max(ah, n);
       float t6v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       if (hi > lo && hi - lo <= D) {  // a pair that observations of this chunk can form
@@ -313,18 +308,14 @@ __global__ void __launch_bounds__(kRpThreads, 8) k_resid_pass(PlanView pv, WorkV
   const float *tcam_buf = wv.tcam + (size_t)wv.lm[b].res_sel * (size_t)pv.O * 6;
   for (int64_t base = ob + (tid & ~31); base < oe; base += blockDim.x) {
     const int64_t o = base + lane;
-    // this observation's pose rows s K of both cameras (zero without a pose term), its
-    // inverse-depth rows, and the weighted linearised residuals w^2 e; each dual is
-    // then formed once as the exact sum of its four products
-    float K[2][2][6], JA[2][2], EW[2][2];
+    // this observation's weighted rows W and its weighted linearised residuals
+    // w r - W (p + dX x_a), p the displacement of its point by the pose step so far; with g = sum W e (exact
+    // four-product sums) its duals are dX . g (landmark) and s [Xp x g; g] (pose pair): the
+    // structure and the rounded rows of the Jacobian pass
+    using M = Num<float>;
+    df g[3], gx[3], vle = df_make(0.f);
 #pragma unroll
-    for (int c2 = 0; c2 < 2; ++c2)
-#pragma unroll
-      for (int r2 = 0; r2 < 2; ++r2) {
-        JA[c2][r2] = EW[c2][r2] = 0.f;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) K[c2][r2][k] = 0.f;
-      }
+    for (int k = 0; k < 3; ++k) g[k] = gx[k] = df_make(0.f);
     int key = -1, slot = -1;
     if (o < oe) {
       slot = pv.obs_slot[o];
@@ -332,60 +323,44 @@ __global__ void __launch_bounds__(kRpThreads, 8) k_resid_pass(PlanView pv, WorkV
       const float4 rl = reinterpret_cast<const float4 *>(res_buf)[o];
       const int a = sm.a[slot];
       const int fw = n - f0;
-      const bool has_pose = n != a;
-      const float sgn = n > a ? 1.f : -1.f;
       const float boost = (prm.near_boost && abs(n - a) < 2) ? 16.f : 1.f;
       const float da = sm.da[slot];
-      const Vec3<float> X = v3<float>(sm.X[slot][0], sm.X[slot][1], sm.X[slot][2]);
-      const Vec3<float> dXda = v3<float>(sm.dX[slot][0], sm.dX[slot][1], sm.dX[slot][2]);
       // point relative to the pair origin (the left centre of frame min(a, n)), the
       // pair's twist (zero without a pose term)
-      const Vec3<float> Xp = v3<float>(X.x + xpo[4 * fw], X.y + xpo[4 * fw + 1], X.z + xpo[4 * fw + 2]);
-      float W[6];
+      df Xp[3];
 #pragma unroll
-      for (int k = 0; k < 6; ++k) W[k] = tws[6 * fw + k];
+      for (int k = 0; k < 3; ++k) Xp[k] = M::shift(sm.X[slot][k], xpo[3 * fw + k]);
+      const float sgn = n > a ? 1.f : -1.f;
+      const float *tw = tws + 6 * fw;
+      const Vec3<float> om = v3<float>(tw[0], tw[1], tw[2]);
+      const Vec3<float> ox = cross(om, v3<float>(Xp[0].h, Xp[1].h, Xp[2].h));
+      const float p[3] = {sgn * (tw[3] + ox.x), sgn * (tw[4] + ox.y), sgn * (tw[5] + ox.z)};  // by the poses
       const float2 *tp = reinterpret_cast<const float2 *>(tcam_buf + (size_t)o * 6);
       const float2 t01 = tp[0], t23 = tp[1], t45 = tp[2];
+      float W[4][3], e[4];
+      const float *Rn = Rw + fw * 18;
+      weighted_rows(prm.loss, lscale, boost, fxs[0], fys[0], Rn, t01.x, t01.y, t23.x, rl.x, rl.y, W, e);
+      weighted_rows(prm.loss, lscale, boost, fxs[1], fys[1], Rn + 9, t23.y, t45.x, t45.y, rl.z, rl.w, W + 2, e + 2);
 #pragma unroll
-      for (int cam = 0; cam < 2; ++cam) {
-        // the camera-frame point as the cost pass at the state formed it (double-float,
-        // rounded once): the same Jacobian the linearisation used
-        const float *Rn = Rw + fw * 18 + cam * 9;
-        const Vec3<float> t = cam ? v3<float>(t23.y, t45.x, t45.y) : v3<float>(t01.x, t01.y, t23.x);
-        const float r0 = cam ? rl.z : rl.x, r1 = cam ? rl.w : rl.y;
-        float rho;
-        const float w2 = boost * robust<float>(prm.loss, lscale, r0 * r0 + r1 * r1, rho);
-        const float fx = fxs[cam], fy = fys[cam], iz = 1.f / t.z;
-        const float j00 = fx * iz, j02 = -fx * t.x * iz * iz, j11 = fy * iz, j12 = -fy * t.y * iz * iz;
-        const Vec3<float> u0 = v3<float>(j00 * Rn[0] + j02 * Rn[2], j00 * Rn[3] + j02 * Rn[5], j00 * Rn[6] + j02 * Rn[8]);
-        const Vec3<float> u1 = v3<float>(j11 * Rn[1] + j12 * Rn[2], j11 * Rn[4] + j12 * Rn[5], j11 * Rn[7] + j12 * Rn[8]);
-        const float ja0 = dot(u0, dXda), ja1 = dot(u1, dXda);
-        float e0 = r0 - ja0 * da, e1 = r1 - ja1 * da;
-        if (has_pose) {
-          const Vec3<float> k0 = cross(Xp, u0), k1 = cross(Xp, u1);
-          K[cam][0][0] = sgn * k0.x; K[cam][0][1] = sgn * k0.y; K[cam][0][2] = sgn * k0.z;
-          K[cam][0][3] = sgn * u0.x; K[cam][0][4] = sgn * u0.y; K[cam][0][5] = sgn * u0.z;
-          K[cam][1][0] = sgn * k1.x; K[cam][1][1] = sgn * k1.y; K[cam][1][2] = sgn * k1.z;
-          K[cam][1][3] = sgn * u1.x; K[cam][1][4] = sgn * u1.y; K[cam][1][5] = sgn * u1.z;
-          float jw0 = 0.f, jw1 = 0.f;
-#pragma unroll
-          for (int k = 0; k < 6; ++k) {
-            jw0 += K[cam][0][k] * W[k];
-            jw1 += K[cam][1][k] * W[k];
-          }
-          e0 -= jw0;
-          e1 -= jw1;
-        }
-        JA[cam][0] = ja0;
-        JA[cam][1] = ja1;
-        EW[cam][0] = w2 * e0;
-        EW[cam][1] = w2 * e1;
+      for (int q = 0; q < 4; ++q) {
+        // the inverse-depth entry W . dX cancels (dX runs along the anchor ray, the rows are
+        // nearly across it): compensated, so that the residual belongs to the same J
+        const float ja = M::round(M::dot(M::of(W[q][0]), M::of(W[q][1]), M::of(W[q][2]), sm.dX[slot][0],
+                                         sm.dX[slot][1], sm.dX[slot][2]));
+        e[q] -= ja * da + (W[q][0] * p[0] + W[q][1] * p[1] + W[q][2] * p[2]);
       }
-      if (has_pose) key = n;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) g[k] = M::sum4(W[0][k], e[0], W[1][k], e[1], W[2][k], e[2], W[3][k], e[3]);
+      vle = M::dot(g[0], g[1], g[2], sm.dX[slot][0], sm.dX[slot][1], sm.dX[slot][2]);
+      if (n != a) {
+        key = n;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) g[k] = M::scale(sgn, g[k]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          gx[k] = M::cross(Xp[(k + 1) % 3], g[(k + 2) % 3], Xp[(k + 2) % 3], g[(k + 1) % 3]);
+      }
     }
-    const df vle =  // this observation's landmark dual
-        slot >= 0 ? sum4_prod(JA[0][0], EW[0][0], JA[0][1], EW[0][1], JA[1][0], EW[1][0], JA[1][1], EW[1][1])
-                  : df_make(0.f);
     {
       // the warp's own landmark accumulators: lanes sharing a landmark (different
       // frames) add in rounds of their rank among those peers, no atomics
@@ -406,20 +381,19 @@ __global__ void __launch_bounds__(kRpThreads, 8) k_resid_pass(PlanView pv, WorkV
     // stage the six pair duals; then 24 lanes, one per (dual, 8-observation segment),
     // each sum their segment's runs of equal target frame and add every run to its
     // pair record (FP64; a run crossing a segment boundary arrives in two parts)
-    float *st = stage + (size_t)warp * 2 * 6 * kRpPitch;
+    df *st = stage + (size_t)warp * 6 * kRpPitch;
     int *keys = sm.key[warp];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      const df v = sum4_prod(K[0][0][k], EW[0][0], K[0][1][k], EW[0][1], K[1][0][k], EW[1][0], K[1][1][k], EW[1][1]);
-      st[(2 * k) * kRpPitch + lane] = v.h;
-      st[(2 * k + 1) * kRpPitch + lane] = v.l;
+    for (int k = 0; k < 3; ++k) {
+      st[k * kRpPitch + lane] = gx[k];
+      st[(3 + k) * kRpPitch + lane] = g[k];
     }
     keys[lane] = key;
     __syncwarp();
     if (__any_sync(0xffffffffu, key >= 0) && lane < 24) {
       const int host_a = sm.a[0];
       const int v = lane % 6, i0 = (lane / 6) * 8;
-      const float *ch = st + (2 * v) * kRpPitch, *cl = st + (2 * v + 1) * kRpPitch;
+      const df *col = st + v * kRpPitch;
       double *rec0 = wv.pdual + (size_t)pv.p_pair_off[b] * 6 + v;
       auto emit = [&](int n, const df_acc &a) {
         const int lo = min(host_a, n), hi = max(host_a, n);
@@ -435,7 +409,7 @@ __global__ void __launch_bounds__(kRpThreads, 8) k_resid_pass(PlanView pv, WorkV
           acc = df_acc();
           cur = k;
         }
-        acc.add(ch[i], cl[i]);
+        M::acc(acc, col[i]);
       }
       if (cur >= 0) emit(cur, acc);
     }

@@ -168,6 +168,9 @@ template <typename T>
 int launch_linearize(const PlanView &pv, const WorkView &wv, const Params &prm, const double *alpha,
                      int cost_only, int gate, void *stream);
 template <typename T>
+int launch_jacobian(const PlanView &pv, const WorkView &wv, const Params &prm, const double *alpha, int gate,
+                    void *stream);
+template <typename T>
 int launch_system(const PlanView &pv, const WorkView &wv, int gate, void *stream);
 template <typename T>
 int launch_schur(const PlanView &pv, const WorkView &wv, const Params &prm, void *stream);
