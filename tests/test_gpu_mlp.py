@@ -163,3 +163,17 @@ def test_controller_features_match_the_lm_state(built_lib, cuda_device):
         assert F[b, 10] == pytest.approx(s["iterations"] / 30.0, abs=1e-6)
         assert F[b, 14] == np.rint(F[b, 14]) and F[b, 14] >= 1.0   # log2 of nu, a power of two
     bs.close()
+
+
+@pytest.mark.parametrize("n", [7, 8, 9, 15, 16, 17, 33, 513])
+def test_gradient_at_cta_edges(built_lib, cuda_device, n):
+    """16 samples a CTA, eight at a time, one partial gradient per further CTA: the edges of
+    those, at the file's tolerances; the scratch is exactly what the header asks for."""
+    theta = M.init(seed=11)
+    X, T = batch(n, 400 + n)
+    ctl = learned.Controller(theta)
+    loss, g = ctl.grad(X, T)
+    ref_loss, ref_g = M.loss_and_grad(theta.astype(np.float64), X.astype(np.float64), T.astype(np.float64))
+    assert abs(loss - ref_loss) / abs(ref_loss) < 1e-5
+    assert rel(g.cpu().numpy(), ref_g) < 1e-4
+    assert rel(ctl.forward(X), M.forward(theta.astype(np.float64), X.astype(np.float64))[0]) < 1e-5
