@@ -10,15 +10,17 @@
 //   k_lg_assemble  row per CTA: the FP32/T copy of S into the factor storage
 //                  (column-major, lower), the exact S (double-float / FP64,
 //                  full, row-major) for the residual, g0 = g - g_L; clears S_L, g_L
-//   per 64-column panel kb:
-//     k_lg_potrf   one CTA factors the 64x64 diagonal block in shared memory,
-//                  16 columns at a time (register-resident 16x16 blocks); on the
-//                  FP32 path k_lg_potrf_rows, one thread per row of the block
+//   per 64-column panel kb (FP32), as far down as the band of S reaches:
+//     k_lg_potrf_rows  one CTA factors the 64x64 diagonal block, one thread per row
 //     k_lg_trsm    thread per row below it: L(i, kb:) = S(i, kb:) L_kk^-T
 //     k_lg_syrk    one CTA per 64x64 tile of the trailing lower triangle,
 //                  C -= L_i L_j^T from shared-memory tiles, 4x4 outputs per thread;
 //                  the next panel's tile column first, then (with the solver's second
-//                  stream) the next k_lg_potrf beside the rest of the update
+//                  stream) the next diagonal block beside the rest of the update
+//   per 32-column panel (FP64):
+//     k_lg_panel   every CTA factors the 32x32 diagonal block, a warp of it solves one
+//                  row below
+//     k_lg_syrk    one CTA per 16x16 tile of the trailing lower triangle
 //   k_lg_fwd/bwd   forward / backward substitution with one CTA per 64-row block,
 //                  chained by per-block flags (32-unknown shuffle chains inside each
 //                  diagonal block, staged in shared memory while the CTA waits its
@@ -28,12 +30,22 @@
 // reduced system (src/Optimization/linear_solvers.cu:195-218).
 #include "kernels.cuh"
 #include "dfloat.cuh"
+#include "chol_subst.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace spgo {
 
-constexpr int kLgNB = 64;
+constexpr int kLgNB = 64;  // rows per block of the substitutions
+
+// Panel width and trailing-update tile.  FP64 issues at 1/64 of the FP32 rate, so one warp
+// instruction holds its quarter of an SM for 64 cycles: FP64 panels are narrow and their work is
+// spread so that a quarter SM has one or two warps of it.
+template <typename T> struct LgShape;
+template <> struct LgShape<float> { static constexpr int NB = 64, TS = 64; };
+template <> struct LgShape<double> { static constexpr int NB = 32, TS = 16; };
+constexpr int kLgPanelRows = 4;  // rows (warps) per CTA of k_lg_panel: a whole 32-byte sector of each column
 
 template <typename T> struct ExactS;
 template <> struct ExactS<float> { using type = float2; };  // (hi, lo) double-float
@@ -80,94 +92,73 @@ __global__ void __launch_bounds__(256) k_lg_assemble(PlanView pv, WorkView wv, i
   }
 }
 
-// One CTA factors the 64x64 diagonal block in shared memory, 16 columns at a time:
-// warp 0 factors each 16x16 diagonal sub-block in registers (lane = row; column k
-// takes one shuffle of the pivot and one per later row), then all threads solve
-// the panel rows below it and update the rest of the panel's lower triangle:
-// three barriers per 16 columns.
-template <typename T>
-__global__ void __launch_bounds__(256) k_lg_potrf(PlanView pv, WorkView wv, int b, int kb) {
+// FP64: one 32-column panel.  Every CTA factors the diagonal block for itself (the chain is the
+// same length for one CTA or for all, and it saves a launch and the block's way through memory),
+// then each warp solves one row below it, lane = column.  Bound by the FP64 pipe of a quarter SM
+// (64 cycles per warp instruction), so the chain is counted in such instructions: column k costs
+// three for 1 / d_k, one for the column of the unit factor U = a(:, k) / d_k and one per column of
+// this warp (j = warp, warp + 4, ..) still to update: 8 on average.  The row solve runs on U too,
+// one FMA per column; 1 / sqrt(d) comes in at the end, for all columns at once.  Measured on a 600-wide system with a band of 245:
+// diagonal blocks and row solves 1354 us in 32-column panels with one CTA and one row per thread
+// (1643 in 64-column ones), 417 us so.
+// The diagonal block is kept as U, which the substitutions read, and 1 / L(k, k); U goes to the
+// transposed place (the upper triangle: other CTAs may still read S_kk).
+__global__ void __launch_bounds__(32 * kLgPanelRows) k_lg_panel(PlanView pv, WorkView wv, int b, int kb) {
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
-  constexpr int kSub = 16;
-  __shared__ T D[kLgNB][kLgNB + 1];
-  __shared__ T di[kLgNB];
-  __shared__ int bad;
-  const int P = 6 * pv.p_npose[b], nb = min(kLgNB, P - kb), tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31;
-  T *fac = reinterpret_cast<T *>(wv.fac) + pv.p_S_off[b];
-  T *dinv = reinterpret_cast<T *>(wv.lg_dinv) + pv.p_param_off[b];
-  for (int idx = tid; idx < nb * nb; idx += blockDim.x) {
-    const int i = idx % nb, j = idx / nb;
-    if (i >= j) D[i][j] = fac[(size_t)(kb + j) * P + kb + i];
+  constexpr int NB = LgShape<double>::NB, W = kLgPanelRows, C = NB / W;
+  static_assert(NB == 32, "lane = row of the diagonal block");
+  __shared__ double col[2][NB], U[NB][NB], dd[NB];
+  const int P = 6 * pv.p_npose[b], nb = min(NB, P - kb), ke = kb + nb;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double *fac = reinterpret_cast<double *>(wv.fac) + pv.p_S_off[b];
+  const int row = ke + blockIdx.x * W + warp;
+  // (rows below exist only under a full panel)
+  double u = row < P ? fac[(size_t)(kb + lane) * P + row] : 0.0;
+  double a[C];  // row `lane` of the block, columns warp + W c (narrow last panel: the identity's beyond nb)
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const int j = warp + W * c;
+    a[c] = (lane < nb && j <= lane) ? fac[(size_t)(kb + j) * P + kb + lane] : (lane == j ? 1.0 : 0.0);
   }
-  if (tid == 0) bad = 0;
+  bool bad = false;
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
+    double *ck = col[k & 1];  // (double-buffered: one barrier per column)
+    if (warp == k % W) ck[lane] = a[k / W];
+    __syncthreads();
+    const double d = ck[k];
+    bad = bad || !(d > 0.0) || !(d < INFINITY);
+    const double t = ck[lane] * rcp_pivot(d);  // rows above k: values nobody reads
+    if (warp == k % W) {
+      U[k][lane] = t;
+      if (lane == 0) dd[k] = d;
+    }
+#pragma unroll
+    for (int c = k / W; c < C; ++c)
+      if (warp + W * c > k) a[c] = fma(-t, ck[warp + W * c], a[c]);
+  }
   __syncthreads();
-  for (int s0 = 0; s0 < nb; s0 += kSub) {
-    const int w = min(kSub, nb - s0), se = s0 + w;
-    if (warp == 0) {
-      T a[kSub];
+  const double y = rsqrt_pivot(dd[lane]);
 #pragma unroll
-      for (int j = 0; j < kSub; ++j) a[j] = (lane < w && j <= lane) ? D[s0 + lane][s0 + j] : T(0);
-      bool badl = false;
-      // (columns k >= w of a narrow last sub-block run on a unit pivot and are discarded)
-#pragma unroll
-      for (int k = 0; k < kSub; ++k) {
-        const T dk = __shfl_sync(0xffffffffu, a[k], k);
-        const T d = k < w ? dk : T(1);
-        badl = badl || !(d > T(0)) || !(d < T(INFINITY));
-        const T lkk = sqrt(d), rinv = T(1) / lkk;
-        const T lik = lane > k ? a[k] * rinv : (lane == k ? lkk : a[k]);
-        a[k] = lik;
-#pragma unroll
-        for (int j = 0; j < kSub; ++j) {
-          const T ljk = __shfl_sync(0xffffffffu, lik, j);
-          if (j > k && lane >= j) a[j] -= lik * ljk;
-        }
-        if (lane == 0 && k < w) di[s0 + k] = rinv;
-      }
-#pragma unroll
-      for (int j = 0; j < kSub; ++j)
-        if (lane < w && j <= lane) D[s0 + lane][s0 + j] = a[j];
-      if (badl && lane == 0) bad = 1;
-    }
-    __syncthreads();
-    // panel rows below the sub-block: L(i, s0:se) = D(i, s0:se) L_sub^-T (right-looking)
-    for (int i = se + tid; i < nb; i += blockDim.x) {
-      T x[kSub];
-#pragma unroll
-      for (int c = 0; c < kSub; ++c) x[c] = c < w ? D[i][s0 + c] : T(0);
-#pragma unroll
-      for (int c = 0; c < kSub; ++c) {
-        x[c] = c < w ? x[c] * di[s0 + c] : T(0);
-#pragma unroll
-        for (int m = c + 1; m < kSub; ++m)
-          if (m < w) x[m] -= x[c] * D[s0 + m][s0 + c];
-      }
-#pragma unroll
-      for (int c = 0; c < kSub; ++c)
-        if (c < w) D[i][s0 + c] = x[c];
-    }
-    __syncthreads();
-    // the rest of the panel: D(i, j) -= sum_c L(i, c) L(j, c) for se <= j <= i < nb
-    const int m = nb - se;
-    for (int idx = tid; idx < m * m; idx += blockDim.x) {
-      const int ii = se + idx % m, jj = se + idx / m;
-      if (ii >= jj) {
-        T acc = T(0);
-#pragma unroll
-        for (int c = 0; c < kSub; ++c)
-          if (c < w) acc += D[ii][s0 + c] * D[jj][s0 + c];
-        D[ii][jj] -= acc;
-      }
-    }
-    __syncthreads();
+  for (int j = 0; j < NB - 1; ++j) {
+    const double uj = __shfl_sync(0xffffffffu, u, j);
+    if (lane > j) u = fma(-uj, U[j][lane], u);
   }
-  if (tid == 0 && bad) atomicOr(&wv.lm[b].fail, FAIL_PIVOT);
-  for (int k = tid; k < nb; k += blockDim.x) dinv[kb + k] = di[k];
-  for (int idx = tid; idx < nb * nb; idx += blockDim.x) {
-    const int i = idx % nb, j = idx / nb;
-    if (i >= j) fac[(size_t)(kb + j) * P + kb + i] = D[i][j];
-  }
+  if (row < P) fac[(size_t)(kb + lane) * P + row] = u * y;
+  if (blockIdx.x != 0) return;
+  for (int i = warp; i < nb; i += W)
+    if (lane < i) fac[(size_t)(kb + i) * P + kb + lane] = U[lane][i];
+  if (warp == 0 && lane < nb) reinterpret_cast<double *>(wv.lg_dinv)[pv.p_param_off[b] + kb + lane] = y;
+  if (threadIdx.x == 0 && bad) atomicOr(&wv.lm[b].fail, FAIL_PIVOT);
+}
+
+// entry i > j of a diagonal block of the substitutions: of the unit factor U(i, j) =
+// L(i, j) / L(j, j) within its 32-wide diagonal parts, of L outside them
+template <typename T>
+__device__ __forceinline__ T lg_diag(const T *L, const T *dinv, int P, int i, int j) {
+  if (i / 32 != j / 32) return L[(size_t)j * P + i];
+  if (std::is_same<T, double>::value) return L[(size_t)i * P + j];  // where k_lg_panel put it
+  return L[(size_t)j * P + i] * dinv[j];
 }
 
 // FP32 path: one CTA of 64 threads factors the 64x64 diagonal block, thread i holding row i of
@@ -176,9 +167,7 @@ __global__ void __launch_bounds__(256) k_lg_potrf(PlanView pv, WorkView wv, int 
 // reads the pivot, and row i > k forms L(i, k) = a(i, k) / L(k, k) and updates its own
 // entries j in (k, i]: a(i, j) -= L(i, k) L(j, k), with L(j, k) taken as a(j, k) from
 // the shared column times 1 / L(k, k).  The serial part per column is one barrier,
-// one square root and one reciprocal; the update is spread over the rows.  (The FP64
-// path keeps k_lg_potrf: FP64 issues at 1/64 of the FP32 rate, and 64 threads carrying
-// the update alone made it slower.)
+// one square root and one reciprocal; the update is spread over the rows.
 __global__ void __launch_bounds__(kLgNB) k_lg_potrf_rows(PlanView pv, WorkView wv, int b, int kb) {
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   __shared__ float col[2][kLgNB];
@@ -223,21 +212,20 @@ __global__ void __launch_bounds__(kLgNB) k_lg_potrf_rows(PlanView pv, WorkView w
 // thread per row below the panel: L(i, kb:ke) = S(i, kb:ke) L_kk^-T, right-looking
 // (once x_j is final it is removed from every later column: independent updates
 // instead of one dependent chain per column)
-template <typename T>
 __global__ void __launch_bounds__(128) k_lg_trsm(PlanView pv, WorkView wv, int b, int kb) {
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
-  __shared__ T D[kLgNB][kLgNB + 1];
-  __shared__ T di[kLgNB];
+  __shared__ float D[kLgNB][kLgNB + 1];
+  __shared__ float di[kLgNB];
   const int P = 6 * pv.p_npose[b], nb = min(kLgNB, P - kb), ke = kb + nb, tid = threadIdx.x;
-  const T *fac_c = reinterpret_cast<const T *>(wv.fac) + pv.p_S_off[b];
-  T *fac = reinterpret_cast<T *>(wv.fac) + pv.p_S_off[b];
-  const T *dinv = reinterpret_cast<const T *>(wv.lg_dinv) + pv.p_param_off[b];
+  const float *fac_c = reinterpret_cast<const float *>(wv.fac) + pv.p_S_off[b];
+  float *fac = reinterpret_cast<float *>(wv.fac) + pv.p_S_off[b];
+  const float *dinv = reinterpret_cast<const float *>(wv.lg_dinv) + pv.p_param_off[b];
   for (int idx0 = tid; idx0 < kLgNB * kLgNB; idx0 += 8 * blockDim.x) {
-    T v[8];
+    float v[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {  // loads first
       const int idx = idx0 + q * blockDim.x, i = idx % kLgNB, j = idx / kLgNB;
-      v[q] = (idx < kLgNB * kLgNB && i > j && i < nb) ? fac_c[(size_t)(kb + j) * P + kb + i] : T(0);
+      v[q] = (idx < kLgNB * kLgNB && i > j && i < nb) ? fac_c[(size_t)(kb + j) * P + kb + i] : 0.f;
     }
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
@@ -245,13 +233,13 @@ __global__ void __launch_bounds__(128) k_lg_trsm(PlanView pv, WorkView wv, int b
       if (idx < kLgNB * kLgNB) D[idx % kLgNB][idx / kLgNB] = v[q];
     }
   }
-  for (int j = tid; j < kLgNB; j += blockDim.x) di[j] = j < nb ? dinv[kb + j] : T(0);
+  for (int j = tid; j < kLgNB; j += blockDim.x) di[j] = j < nb ? dinv[kb + j] : 0.f;
   __syncthreads();
   const int i = ke + blockIdx.x * blockDim.x + tid;
   if (i >= P) return;
-  T x[kLgNB];
+  float x[kLgNB];
 #pragma unroll
-  for (int j = 0; j < kLgNB; ++j) x[j] = j < nb ? fac_c[(size_t)(kb + j) * P + i] : T(0);
+  for (int j = 0; j < kLgNB; ++j) x[j] = j < nb ? fac_c[(size_t)(kb + j) * P + i] : 0.f;
 #pragma unroll
   for (int j = 0; j < kLgNB; ++j) {
     x[j] *= di[j];
@@ -268,17 +256,13 @@ __global__ void __launch_bounds__(128) k_lg_trsm(PlanView pv, WorkView wv, int b
 template <typename T>
 __global__ void __launch_bounds__(256) k_lg_syrk(PlanView pv, WorkView wv, int b, int kb, int mode) {
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
-  __shared__ T LR[kLgNB][kLgNB + 1];
-  __shared__ T LC[kLgNB][kLgNB + 1];
-  const int P = 6 * pv.p_npose[b], nb = min(kLgNB, P - kb), ke = kb + nb, tid = threadIdx.x;
-  // tile t -> (ti >= tj) of the trailing lower triangle (mode 2: of the triangle without
-  // its first tile column, shifted by one)
-  const int t = blockIdx.x;
-  int ti, tj;
-  if (mode == 1) {
-    ti = t;
-    tj = 0;
-  } else {
+  constexpr int NB = LgShape<T>::NB, TS = LgShape<T>::TS, R = TS / 16;
+  __shared__ T LR[NB][TS + 1];
+  __shared__ T LC[NB][TS + 1];
+  const int P = 6 * pv.p_npose[b], nb = min(NB, P - kb), ke = kb + nb, tid = threadIdx.x;
+  // tile t -> (ti >= tj)
+  int t = blockIdx.x, ti = t, tj = 0;
+  if (mode != 1) {
     ti = (int)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
     while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
     while (ti * (ti + 1) / 2 > t) --ti;
@@ -288,36 +272,36 @@ __global__ void __launch_bounds__(256) k_lg_syrk(PlanView pv, WorkView wv, int b
       ++tj;
     }
   }
-  const int R0 = ke + kLgNB * ti, C0 = ke + kLgNB * tj;
+  const int R0 = ke + TS * ti, C0 = ke + TS * tj;
   T *fac = reinterpret_cast<T *>(wv.fac) + pv.p_S_off[b];
-  for (int idx = tid; idx < nb * kLgNB; idx += blockDim.x) {
-    const int r = idx % kLgNB, k = idx / kLgNB;
+  for (int idx = tid; idx < nb * TS; idx += blockDim.x) {
+    const int r = idx % TS, k = idx / TS;
     LR[k][r] = R0 + r < P ? fac[(size_t)(kb + k) * P + R0 + r] : T(0);
     LC[k][r] = C0 + r < P ? fac[(size_t)(kb + k) * P + C0 + r] : T(0);
   }
   __syncthreads();
   const int tx = tid % 16, ty = tid / 16;
-  T acc[4][4];
+  T acc[R][R];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < R; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = T(0);
+    for (int j = 0; j < R; ++j) acc[i][j] = T(0);
   for (int k = 0; k < nb; ++k) {
-    T a[4], c[4];
+    T a[R], c[R];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < R; ++i) {
       a[i] = LR[k][tx + 16 * i];
       c[i] = LC[k][ty + 16 * i];
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < R; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] += a[i] * c[j];
+      for (int j = 0; j < R; ++j) acc[i][j] += a[i] * c[j];
   }
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
+  for (int j = 0; j < R; ++j)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < R; ++i) {
       const int r = R0 + tx + 16 * i, c = C0 + ty + 16 * j;
       if (r < P && c < P && r >= c) fac[(size_t)c * P + r] -= acc[i][j];
     }
@@ -358,7 +342,9 @@ __global__ void __launch_bounds__(256) k_lg_fwd(PlanView pv, WorkView wv, int b,
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   __shared__ T part[4][kLgNB];
   __shared__ T zs[kLgNB];
-  __shared__ T Ld[kLgNB][kLgNB + 1];  // the diagonal block (lower, zero elsewhere) and its pivots,
+  // the diagonal block (strictly lower, its two 32-wide diagonal parts of the unit factor, so that
+  // the chain is one shuffle and one FMA per unknown) and the pivots' reciprocals,
+  __shared__ T Ld[kLgNB][kLgNB + 1];
   __shared__ T ds[kLgNB];             // staged while the earlier blocks are still being solved
   __shared__ int timed_out;
   const int P = 6 * pv.p_npose[b], po = pv.p_param_off[b];
@@ -373,12 +359,13 @@ __global__ void __launch_bounds__(256) k_lg_fwd(PlanView pv, WorkView wv, int b,
   if (tid == 0) timed_out = 0;
   for (int idx = tid; idx < kLgNB * kLgNB; idx += blockDim.x) {
     const int i = idx % kLgNB, j = idx / kLgNB;
-    Ld[i][j] = (i < nb && j <= i) ? Lat(kb + i, kb + j) : T(0);
+    Ld[i][j] = (i < nb && j < i) ? lg_diag(L, dinv, P, kb + i, kb + j) : T(0);
   }
   if (tid < kLgNB) ds[tid] = tid < nb ? dinv[kb + tid] : T(0);
   __syncthreads();
   T acc = T(0);
-  for (int j = 0; j < k; ++j) {  // earlier blocks are full 64-wide
+  const int bw = 6 * pv.p_pair_D[b] - 1;  // L(i, j) = 0 for i - j > bw
+  for (int j = max(0, kb - bw) / kLgNB; j < k; ++j) {  // earlier blocks are full 64-wide
     // this block's part of L is loaded before the wait for block j's solution
     const int c0 = j * kLgNB + 16 * q;
     T lv[16];
@@ -419,20 +406,12 @@ __global__ void __launch_bounds__(256) k_lg_fwd(PlanView pv, WorkView wv, int b,
         }
         v += (v1 + v2) + v3;
       }
-      T lr[32], di[32];
+      T lr[32];
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        lr[c] = (lane < w && c < lane) ? Ld[h + lane][h + c] : T(0);
-        di[c] = c < w ? ds[h + c] : T(0);
-      }
+      for (int c = 0; c < 32; ++c) lr[c] = Ld[h + lane][h + c];
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        T yc = v * di[c];
-        yc = __shfl_sync(0xffffffffu, yc, c);
-        if (lane == c) v = yc;
-        v -= lr[c] * yc;
-      }
-      if (lane < w) zs[h + lane] = v;
+      for (int c = 0; c < 31; ++c) v -= lr[c] * __shfl_sync(0xffffffffu, v, c);
+      if (lane < w) zs[h + lane] = v * ds[h + lane];
       __syncwarp();
     }
   }
@@ -455,7 +434,9 @@ __global__ void __launch_bounds__(256) k_lg_bwd(PlanView pv, WorkView wv, int b,
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   __shared__ T part[4][kLgNB];
   __shared__ T zs[kLgNB];
-  __shared__ T Ld[kLgNB][kLgNB + 1];  // the diagonal block (lower, zero elsewhere) and its pivots,
+  // the diagonal block (strictly lower, its two 32-wide diagonal parts of the unit factor, so that
+  // the chain is one shuffle and one FMA per unknown) and the pivots' reciprocals,
+  __shared__ T Ld[kLgNB][kLgNB + 1];
   __shared__ T ds[kLgNB];             // staged while the later blocks are still being solved
   __shared__ int timed_out;
   const int P = 6 * pv.p_npose[b], po = pv.p_param_off[b];
@@ -471,12 +452,13 @@ __global__ void __launch_bounds__(256) k_lg_bwd(PlanView pv, WorkView wv, int b,
   if (tid == 0) timed_out = 0;
   for (int idx = tid; idx < kLgNB * kLgNB; idx += blockDim.x) {
     const int i = idx % kLgNB, j = idx / kLgNB;
-    Ld[i][j] = (i < nb && j <= i) ? Lat(kb + i, kb + j) : T(0);
+    Ld[i][j] = (i < nb && j < i) ? lg_diag(L, dinv, P, kb + i, kb + j) : T(0);
   }
   if (tid < kLgNB) ds[tid] = tid < nb ? dinv[kb + tid] : T(0);
   __syncthreads();
   T acc = T(0);
-  for (int j = nblk - 1; j > k; --j) {  // later blocks, finished by lower-numbered CTAs
+  const int bw = 6 * pv.p_pair_D[b] - 1;
+  for (int j = min(nblk - 1, (kb + nb - 1 + bw) / kLgNB); j > k; --j) {  // later blocks, finished by lower-numbered CTAs
     // this block's part of L is loaded before the wait for block j's solution
     const int jb = j * kLgNB, nbj = min(kLgNB, P - jb);
     T lv[16];
@@ -520,19 +502,12 @@ __global__ void __launch_bounds__(256) k_lg_bwd(PlanView pv, WorkView wv, int b,
         }
         v += (v1 + v2) + v3;
       }
-      T lc[32], di[32];  // column `lane` of the diagonal block, pivots
+      T lc[32];  // column `lane` of the diagonal block
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        lc[c] = (c < w && lane < c) ? Ld[h + c][h + lane] : T(0);
-        di[c] = c < w ? ds[h + c] : T(0);
-      }
+      for (int c = 0; c < 32; ++c) lc[c] = Ld[h + c][h + lane];
+      v *= ds[h + lane];  // U^T x = L_jj^-1 (..)
 #pragma unroll
-      for (int c = 31; c >= 0; --c) {
-        T xc = v * di[c];
-        xc = __shfl_sync(0xffffffffu, xc, c);
-        if (lane == c) v = xc;
-        v -= lc[c] * xc;
-      }
+      for (int c = 31; c > 0; --c) v -= lc[c] * __shfl_sync(0xffffffffu, v, c);
       if (lane < w) zs[h + lane] = v;
       __syncwarp();
     }
@@ -629,45 +604,49 @@ int launch_factor_large(const PlanView &pv, const WorkView &wv, const Params &pr
   const uint64_t wait_ns = wait_limit_ns(prm);
   k_lg_assemble<T><<<P, 256, 0, st>>>(pv, wv, b);
   int n = 1;
-  auto potrf = [&](int kb, cudaStream_t on) {
-    if constexpr (std::is_same<T, float>::value)
-      k_lg_potrf_rows<<<1, kLgNB, 0, on>>>(pv, wv, b, kb);
-    else
-      k_lg_potrf<T><<<1, 256, 0, on>>>(pv, wv, b, kb);
-    ++n;
-  };
-  // one panel of look-ahead: once panel kb's rows are solved, the next panel's columns take
-  // its update first and the next diagonal block is factored on the side stream while the
-  // rest of the trailing matrix is updated; every element takes the same updates in the
-  // same order as without it
-  cudaStream_t sd = (cudaStream_t)side;
-  cudaEvent_t ea = (cudaEvent_t)ev_a, eb = (cudaEvent_t)ev_b;
-  const bool ahead = sd && ea && eb;
-  potrf(0, st);
-  for (int kb = 0; kb < P; kb += kLgNB) {
-    const int ke = min(P, kb + kLgNB);
-    if (ke >= P) break;  // (the last diagonal block is factored: nothing below it)
-    const int M = P - ke, nt = (M + kLgNB - 1) / kLgNB;
-    k_lg_trsm<T><<<(M + 127) / 128, 128, 0, st>>>(pv, wv, b, kb);
-    n += 1;
-    if (!ahead) {
-      k_lg_syrk<T><<<nt * (nt + 1) / 2, 256, 0, st>>>(pv, wv, b, kb, 0);
+  constexpr int NB = LgShape<T>::NB, TS = LgShape<T>::TS;
+  const int bw = 6 * D - 1;  // S and L are zero beyond it: a panel reaches bw rows down
+  if constexpr (std::is_same<T, double>::value) {
+    for (int kb = 0; kb < P; kb += NB) {
+      const int M = std::min(std::max(P - kb - NB, 0), bw), nt = (M + TS - 1) / TS;
+      k_lg_panel<<<std::max(1, (M + kLgPanelRows - 1) / kLgPanelRows), 32 * kLgPanelRows, 0, st>>>(pv, wv, b, kb);
       ++n;
-      potrf(ke, st);
-      continue;
+      if (nt > 0) {
+        k_lg_syrk<T><<<nt * (nt + 1) / 2, 256, 0, st>>>(pv, wv, b, kb, 0);
+        ++n;
+      }
     }
-    k_lg_syrk<T><<<nt, 256, 0, st>>>(pv, wv, b, kb, 1);
+  } else {
+    // one panel of look-ahead: once panel kb's rows are solved, the next panel's columns take
+    // its update first and the next diagonal block is factored on the side stream while the
+    // rest of the trailing matrix is updated; every element takes the same updates in the
+    // same order as without it
+    cudaStream_t sd = (cudaStream_t)side;
+    cudaEvent_t ea = (cudaEvent_t)ev_a, eb = (cudaEvent_t)ev_b;
+    const bool ahead = sd && ea && eb;
+    k_lg_potrf_rows<<<1, kLgNB, 0, st>>>(pv, wv, b, 0);
     ++n;
-    cudaError_t e = cudaEventRecord(ea, st);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(sd, ea, 0);
-    if (e != cudaSuccess) return (int)e;
-    potrf(ke, sd);
-    if ((e = cudaEventRecord(eb, sd)) != cudaSuccess) return (int)e;
-    if (nt > 1) {
-      k_lg_syrk<T><<<(nt - 1) * nt / 2, 256, 0, st>>>(pv, wv, b, kb, 2);
-      ++n;
+    for (int kb = 0; kb + NB < P; kb += NB) {
+      const int ke = kb + NB, M = std::min(P - ke, bw), nt = (M + TS - 1) / TS;
+      k_lg_trsm<<<(M + 127) / 128, 128, 0, st>>>(pv, wv, b, kb);
+      n += 3;
+      if (!ahead) {
+        k_lg_syrk<T><<<nt * (nt + 1) / 2, 256, 0, st>>>(pv, wv, b, kb, 0);
+        k_lg_potrf_rows<<<1, kLgNB, 0, st>>>(pv, wv, b, ke);
+        continue;
+      }
+      k_lg_syrk<T><<<nt, 256, 0, st>>>(pv, wv, b, kb, 1);
+      cudaError_t e = cudaEventRecord(ea, st);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(sd, ea, 0);
+      if (e != cudaSuccess) return (int)e;
+      k_lg_potrf_rows<<<1, kLgNB, 0, sd>>>(pv, wv, b, ke);
+      if ((e = cudaEventRecord(eb, sd)) != cudaSuccess) return (int)e;
+      if (nt > 1) {
+        k_lg_syrk<T><<<nt * (nt - 1) / 2, 256, 0, st>>>(pv, wv, b, kb, 2);
+        ++n;
+      }
+      if ((e = cudaStreamWaitEvent(st, eb, 0)) != cudaSuccess) return (int)e;
     }
-    if ((e = cudaStreamWaitEvent(st, eb, 0)) != cudaSuccess) return (int)e;
   }
   const int nblk = (P + kLgNB - 1) / kLgNB;
   int *ff = wv.lg_flag + param_off, *fb = wv.lg_flag + pv.total_params + param_off;

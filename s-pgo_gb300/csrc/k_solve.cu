@@ -36,7 +36,12 @@ __device__ __forceinline__ T s_entry(const T *A, const T *SL, int P, int r, int 
 // factorises the 16x16 diagonal block, all threads solve the rows below it
 // (independent per row) and apply the rank-16 trailing update, the next block's
 // columns first, so that warp 0 factorises the next diagonal block while the other
-// warps update the rest (one block of look-ahead); three barriers per block.  The substitutions are blocked the same way (two barriers per
+// warps update the rest (one block of look-ahead); three barriers per block.
+// Bound by the diagonal blocks' chain in FP32 (one 16-pose window: 35 us with a pivot, its
+// correctly rounded root and reciprocal and fifteen shuffles per column, 29.7 us in groups of
+// four columns) and in FP64 by the FP64 pipe's 2 FMA per cycle and SM (eight solves of a window
+// of up to 16 poses: 613 us with a thread per row, a warp per two columns and a row's columns
+// in one lane; 377 us with the work laid out by FP64 instructions as below).  The substitutions are blocked the same way (two barriers per
 // block).  `refine` iterative-refinement steps form the residual g_S - S x
 // (double-float on the FP32 path, FP64 otherwise) from A and S_L in one
 // coalesced pass over the lower triangle.  Clears the S_L / g_L tiles it consumed.
@@ -85,35 +90,93 @@ __device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *
     x[i] = 0.0;
   }
   if (tid == 0) *fail_s = 0;
+  __shared__ int drawn;  // FP64: elements of the trailing update handed out
   __syncthreads();
   // warp 0: the diagonal block [kb, kb + kPanel) in registers; lane i < w holds row i
-  // (a[j] = L(kb+i, kb+j), j <= i); column k is finished with one shuffle of the pivot
-  // and one per later row
+  // (a[j] = L(kb+i, kb+j), j <= i; rows past the last block's w are the identity's).
+  // FP32: four columns at a time, their 4x4 pivot block factored by every lane from ten
+  // shuffles, its rows then exchanged through shared memory, so that the chain holds one
+  // exchange per four columns.  FP64, where one instruction of the warp takes 64 cycles: lane
+  // (i, h) holds row i's columns of parity h, and a column costs three for 1 / d, one for its
+  // column of the unit factor U = a / d and one per two later columns; 1 / sqrt(d) for all
+  // columns at once at the end (133 instructions a block; 330 with a row's 16 columns in a lane
+  // and the library's square root and reciprocal).  The block keeps U, for the row solves and
+  // the substitutions.
   auto factor_diag = [&](int kb) {
     const int w = min(kb + kPanel, P) - kb;
-    T a[kPanel];
-#pragma unroll
-    for (int j = 0; j < kPanel; ++j) a[j] = (lane < w && j <= lane) ? Lm[ix(kb + lane, kb + j)] : T(0);
     bool bad = false;
-    // (columns k >= w of a narrow last block run on a unit pivot and are discarded)
+    if constexpr (std::is_same<T, float>::value) {
+      float a[kPanel];
 #pragma unroll
-    for (int k = 0; k < kPanel; ++k) {
-      const T dk = __shfl_sync(0xffffffffu, a[k], k);
-      const T d = k < w ? dk : T(1);
-      bad = bad || !(d > T(0)) || !(d < T(INFINITY));  // (no FP64 conversion on the pivot chain)
-      const T lkk = sqrt(d), rinv = T(1) / lkk;  // correctly rounded: the refinement step relies on it
-      const T lik = lane > k ? a[k] * rinv : (lane == k ? lkk : a[k]);
-      a[k] = lik;
+      for (int j = 0; j < kPanel; ++j)
+        a[j] = (lane < w && j <= lane) ? Lm[ix(kb + lane, kb + j)] : (lane == j ? 1.f : 0.f);
+      __shared__ __align__(16) float rows[2][4 * kPanel];
+      auto rsq = [&](float d) {  // NaN unless 0 < d < inf
+        float r = rsqrtf(d);
+        r = fmaf(0.5f * r, fmaf(-d * r, r, 1.f), r);
+        bad = bad || !(r > 0.f);
+        return r;
+      };
 #pragma unroll
-      for (int j = 0; j < kPanel; ++j) {
-        const T ljk = __shfl_sync(0xffffffffu, lik, j);
-        if (j > k && lane >= j) a[j] -= lik * ljk;
+      for (int k = 0; k < kPanel; k += 4) {
+        float p[4][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int s = 0; s <= q; ++s) p[q][s] = __shfl_sync(0xffffffffu, a[k + s], k + q);
+        const float r0 = rsq(p[0][0]);
+        const float l10 = p[1][0] * r0, l20 = p[2][0] * r0, l30 = p[3][0] * r0;
+        const float r1 = rsq(fmaf(-l10, l10, p[1][1]));
+        const float l21 = fmaf(-l20, l10, p[2][1]) * r1, l31 = fmaf(-l30, l10, p[3][1]) * r1;
+        const float r2 = rsq(fmaf(-l21, l21, fmaf(-l20, l20, p[2][2])));
+        const float l32 = fmaf(-l31, l21, fmaf(-l30, l20, p[3][2])) * r2;
+        const float r3 = rsq(fmaf(-l32, l32, fmaf(-l31, l31, fmaf(-l30, l30, p[3][3]))));
+        // this row's entries of the four columns (rows above them compute values nobody reads)
+        a[k] *= r0;
+        a[k + 1] = fmaf(-a[k], l10, a[k + 1]) * r1;
+        a[k + 2] = fmaf(-a[k + 1], l21, fmaf(-a[k], l20, a[k + 2])) * r2;
+        a[k + 3] = fmaf(-a[k + 2], l32, fmaf(-a[k + 1], l31, fmaf(-a[k], l30, a[k + 3]))) * r3;
+        if (lane < 4 && k + lane < w) dinv[kb + k + lane] = lane == 0 ? r0 : lane == 1 ? r1 : lane == 2 ? r2 : r3;
+        if (k + 4 < kPanel) {
+          float *xk = rows[(k >> 2) & 1];  // (double-buffered: one warp barrier per four columns)
+          if (lane < kPanel)
+            *reinterpret_cast<float4 *>(xk + 4 * lane) = make_float4(a[k], a[k + 1], a[k + 2], a[k + 3]);
+          __syncwarp();
+#pragma unroll
+          for (int j = k + 4; j < kPanel; ++j) {
+            const float4 v = *reinterpret_cast<const float4 *>(xk + 4 * j);
+            a[j] = fmaf(-a[k + 3], v.w, fmaf(-a[k + 2], v.z, fmaf(-a[k + 1], v.y, fmaf(-a[k], v.x, a[j]))));
+          }
+        }
       }
-      if (lane == 0 && k < w) dinv[kb + k] = rinv;
-    }
 #pragma unroll
-    for (int j = 0; j < kPanel; ++j)
-      if (lane < w && j <= lane) Lm[ix(kb + lane, kb + j)] = a[j];
+      for (int j = 0; j < kPanel; ++j)
+        if (lane < w && j <= lane) Lm[ix(kb + lane, kb + j)] = a[j];
+    } else {
+      const int i = lane & 15, h = lane >> 4;
+      double a[kPanel / 2], dk = 1.0;
+#pragma unroll
+      for (int c = 0; c < kPanel / 2; ++c) {
+        const int j = 2 * c + h;
+        a[c] = (i < w && j <= i) ? Lm[ix(kb + i, kb + j)] : (i == j ? 1.0 : 0.0);
+      }
+#pragma unroll
+      for (int k = 0; k < kPanel; ++k) {
+        const int from = 16 * (k & 1);  // the half that holds column k
+        const double d = __shfl_sync(0xffffffffu, a[k / 2], k + from);
+        bad = bad || !(d > 0.0) || !(d < INFINITY);
+        if (lane == k) dk = d;
+        const double t = __shfl_sync(0xffffffffu, a[k / 2], i + from) * rcp_pivot(d);
+        if (h == 0 && i > k && i < w) Lm[ix(kb + i, kb + k)] = t;
+#pragma unroll
+        for (int c = (k + 1) / 2; c < kPanel / 2; ++c) {
+          const double ajk = __shfl_sync(0xffffffffu, a[k / 2], 2 * c + h + from);
+          if (2 * c + h > k) a[c] = fma(-t, ajk, a[c]);  // (rows above k: values nobody reads)
+        }
+      }
+      const double y = rsqrt_pivot(dk);  // lane = column
+      if (lane < w) dinv[kb + lane] = y;
+    }
     if (bad && lane == 0) *fail_s = 1;
   };
   // the update of columns [c0, c1) (rows i >= j) with the finished block kb: warp wi of
@@ -155,36 +218,92 @@ __device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *
   for (int kb = 0; kb < P; kb += kPanel) {
     const int ke = min(kb + kPanel, P), w = ke - kb;
     // rows below the block: L(i, kb:ke) = S(i, kb:ke) L_D^-T
-    int cbk[kPanel];
+    if constexpr (std::is_same<T, double>::value) {
+      if (ke >= P) break;  // (rows below exist only under a full block)
+      // four lanes per row, lane q holding columns q, q + 4, ..: 36 + 4 FP64 instructions a warp
+      // however few rows are left (136 with a thread per row)
+      const int q = lane & 3;
+      for (int i0 = ke + 8 * warp; i0 < P; i0 += 8 * nw) {
+        const int i = i0 + (lane >> 2);
+        double u[4];
 #pragma unroll
-    for (int c = 0; c < kPanel; ++c) cbk[c] = c < w ? cb[kb + c] : 0;
-    for (int i = ke + tid; i < P; i += nt) {
-      T r[kPanel];
+        for (int c = 0; c < 4; ++c) u[c] = i < P ? Lm[ix(i, kb + q + 4 * c)] : 0.0;
 #pragma unroll
-      for (int c = 0; c < kPanel; ++c) r[c] = c < w ? Lm[cbk[c] + i] : T(0);
+        for (int j = 0; j < kPanel - 1; ++j) {
+          const double uj = __shfl_sync(0xffffffffu, u[j / 4], (lane & ~3) | (j & 3));
 #pragma unroll
-      for (int c = 0; c < kPanel; ++c) {
-        if (c < w) {
-          T v = r[c];
-#pragma unroll
-          for (int m = 0; m < c; ++m) v -= r[m] * Lm[ix(kb + c, kb + m)];
-          r[c] = v * dinv[kb + c];
+          for (int c = (j + 1) / 4; c < 4; ++c)
+            if (q + 4 * c > j) u[c] = fma(-uj, Lm[ix(kb + q + 4 * c, kb + j)], u[c]);
         }
-      }
 #pragma unroll
-      for (int c = 0; c < kPanel; ++c)
-        if (c < w) Lm[cbk[c] + i] = r[c];
+        for (int c = 0; c < 4; ++c)
+          if (i < P) Lm[ix(i, kb + q + 4 * c)] = u[c] * dinv[kb + q + 4 * c];
+      }
+      // trailing update, an element of the packed triangle per lane, so that no lane idles at the
+      // columns' ends (a warp per two columns kept 40 to 75 % of them busy); behind the next
+      // block's columns the warps draw 32 elements at a time, warp 0 once it has factored
+      const int R = P - ke, n = R * (R + 1) / 2, w2 = min(kPanel, R), n1 = w2 * R - w2 * (w2 - 1) / 2;
+      T *tri = Lm + ix(ke, ke);
+      int cbk[kPanel];
+#pragma unroll
+      for (int c = 0; c < kPanel; ++c) cbk[c] = cb[kb + c];
+      auto update = [&](int o) {
+        const int r = n - 1 - o;  // from the end: column P - 1 - jj holds jj + 1 elements
+        int jj = (int)((sqrtf(8.f * (float)r + 1.f) - 1.f) * 0.5f);
+        jj += (jj + 1) * (jj + 2) / 2 <= r;
+        jj -= jj * (jj + 1) / 2 > r;
+        const int j = P - 1 - jj, i = P - 1 - (r - jj * (jj + 1) / 2);
+        double a0 = 0.0, a1 = 0.0;
+#pragma unroll
+        for (int k = 0; k < kPanel; k += 2) {
+          a0 += Lm[cbk[k] + i] * Lm[cbk[k] + j];
+          a1 += Lm[cbk[k + 1] + i] * Lm[cbk[k + 1] + j];
+        }
+        tri[o] -= a0 + a1;
+      };
+      __syncthreads();
+      for (int o = tid; o < n1; o += nt) update(o);
+      if (tid == 0) drawn = n1;
+      __syncthreads();
+      if (warp == 0) factor_diag(ke);
+      for (;;) {
+        int o = 0;
+        if (lane == 0) o = atomicAdd(&drawn, 32);
+        o = __shfl_sync(0xffffffffu, o, 0);
+        if (o >= n) break;
+        if (o + lane < n) update(o + lane);
+      }
+    } else {
+      int cbk[kPanel];
+#pragma unroll
+      for (int c = 0; c < kPanel; ++c) cbk[c] = c < w ? cb[kb + c] : 0;
+      for (int i = ke + tid; i < P; i += nt) {
+        T r[kPanel];
+#pragma unroll
+        for (int c = 0; c < kPanel; ++c) r[c] = c < w ? Lm[cbk[c] + i] : T(0);
+#pragma unroll
+        for (int c = 0; c < kPanel; ++c) {
+          if (c < w) {
+            T v = r[c];
+#pragma unroll
+            for (int m = 0; m < c; ++m) v -= r[m] * Lm[ix(kb + c, kb + m)];
+            r[c] = v * dinv[kb + c];
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < kPanel; ++c)
+          if (c < w) Lm[cbk[c] + i] = r[c];
+      }
+      __syncthreads();
+      if (ke >= P) break;
+      const int ke2 = min(ke + kPanel, P);
+      update_cols(std::integral_constant<int, 2>{}, cbk, w, ke, ke2, warp, nw);  // the next block's columns
+      __syncthreads();
+      if (warp == 0)
+        factor_diag(ke);
+      else
+        update_cols(std::integral_constant<int, 4>{}, cbk, w, ke2, P, warp - 1, nw - 1);
     }
-    __syncthreads();
-    if (ke >= P) break;
-    const int ke2 = min(ke + kPanel, P);
-    update_cols(std::integral_constant<int, 2>{}, cbk, w, ke, ke2, warp, nw);  // the next block's columns
-    __syncthreads();
-    // (4 columns per pass in FP32, 2 in FP64 to bound registers)
-    if (warp == 0)
-      factor_diag(ke);
-    else
-      update_cols(std::integral_constant<int, sizeof(T) == 8 ? 2 : 4>{}, cbk, w, ke2, P, warp - 1, nw - 1);
     __syncthreads();
     if (*fail_s) return;
   }
