@@ -30,66 +30,100 @@
 namespace spgo {
 
 // ---- global poses: G[0] = I, G[k+1] = G[k] inv(T_k); right camera G T_r_to_l ----
-// One warp per problem: an inclusive shuffle scan of the 3x4 products (FP64),
-// 32 frames per pass with the running prefix carried between passes
-// (the reference walks the chain with one thread, Solver_cuda.cu:472-491).
-__device__ __forceinline__ void write_frame(const WorkView &wv, size_t f, const double *G, const double *Trl) {
-  double Gr[12];
-  compose34(G, Trl, Gr);
+// FP64 path.  One CTA per problem: an inclusive scan of the 3x4 products in shared memory, three
+// threads (rows) per frame, blockDim / 3 frames per pass with the running prefix carried between
+// passes (the reference walks the chain with one thread, Solver_cuda.cu:472-491).  Bound by the
+// scan's FP64 instructions, 64 cycles each for a quarter of an SM: a row's product takes 12, where
+// a lane per frame took 36 and 32 frames shared one quarter of the SM (100 poses: 57 us, 17.3
+// us so; 10 poses: 18.6 and 8.5 us).
+constexpr int kChainFrames = 128;
+
+// row r of frame f, G its 3x4 pose
+__device__ __forceinline__ void write_frame_row(const WorkView &wv, size_t f, int r, const double *G, const double *Trl) {
+  double Gr[4];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
+  for (int j = 0; j < 4; ++j) Gr[j] = G[0] * Trl[j] + G[1] * Trl[4 + j] + G[2] * Trl[8 + j];
+  Gr[3] += G[3];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      wv.fr_Rd[f * 18 + 3 * i + j] = G[4 * i + j];
-      wv.fr_Rd[f * 18 + 9 + 3 * i + j] = Gr[4 * i + j];
-      const float gl = (float)G[4 * i + j], gr = (float)Gr[4 * i + j];
-      wv.fr_Rf[f * 18 + 3 * i + j] = gl;
-      wv.fr_Rf[f * 18 + 9 + 3 * i + j] = gr;
-      wv.fr_Rl[f * 18 + 3 * i + j] = (float)(G[4 * i + j] - (double)gl);
-      wv.fr_Rl[f * 18 + 9 + 3 * i + j] = (float)(Gr[4 * i + j] - (double)gr);
-    }
-    const double cl = G[4 * i + 3], cr = Gr[4 * i + 3];
-    wv.fr_c[f * 6 + i] = cl;
-    wv.fr_c[f * 6 + 3 + i] = cr;
-    const float hl = (float)cl, hr = (float)cr;
-    wv.fr_ch[f * 6 + i] = hl;
-    wv.fr_ch[f * 6 + 3 + i] = hr;
-    wv.fr_cl[f * 6 + i] = (float)(cl - (double)hl);
-    wv.fr_cl[f * 6 + 3 + i] = (float)(cr - (double)hr);
+  for (int j = 0; j < 3; ++j) {
+    const size_t q = f * 18 + 3 * r + j;
+    wv.fr_Rd[q] = G[j];
+    wv.fr_Rd[q + 9] = Gr[j];
+    const float gl = (float)G[j], gr = (float)Gr[j];
+    wv.fr_Rf[q] = gl;
+    wv.fr_Rf[q + 9] = gr;
+    wv.fr_Rl[q] = (float)(G[j] - (double)gl);
+    wv.fr_Rl[q + 9] = (float)(Gr[j] - (double)gr);
   }
+  const size_t q = f * 6 + r;
+  wv.fr_c[q] = G[3];
+  wv.fr_c[q + 3] = Gr[3];
+  const float hl = (float)G[3], hr = (float)Gr[3];
+  wv.fr_ch[q] = hl;
+  wv.fr_ch[q + 3] = hr;
+  wv.fr_cl[q] = (float)(G[3] - (double)hl);
+  wv.fr_cl[q + 3] = (float)(Gr[3] - (double)hr);
 }
 
-__global__ void k_chain(PlanView pv, WorkView wv, const double *__restrict__ poses, int gate) {
-  const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (b >= pv.B) return;
+// row p of a product P M of 3x4 poses
+__device__ __forceinline__ void compose_row(const double *p, const double *M, double *o) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) o[j] = p[0] * M[j] + p[1] * M[4 + j] + p[2] * M[8 + j];
+  o[3] += p[3];
+}
+
+__global__ void __launch_bounds__(3 * kChainFrames) k_chain(PlanView pv, WorkView wv, const double *__restrict__ poses,
+                                                            int gate) {
+  const int b = blockIdx.x;
   if (!problem_active(wv.lm, b, gate)) return;
+  __shared__ double buf[2][kChainFrames][12];
+  __shared__ double last[12];
   const int N = pv.p_npose[b], fo = pv.p_frame_off[b], po = pv.p_pose_off[b];
+  const int nf = blockDim.x / 3, f = threadIdx.x / 3, r = threadIdx.x % 3;
   const double *Trl = pv.p_Trl + 12 * b;
-  double carry[12] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0};
-  if (lane == 0) write_frame(wv, (size_t)fo, carry, Trl);
-  for (int s = 0; s < N; s += 32) {
-    const int k = s + lane;
-    double M[12] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0};
-    if (k < N) invert34(poses + 12 * (size_t)(po + k), M);
-    // inclusive scan: M_k <- M_0 M_1 ... M_k (earlier factors on the left)
+  if (f == 0) {
+    const double I[4] = {r == 0 ? 1.0 : 0.0, r == 1 ? 1.0 : 0.0, r == 2 ? 1.0 : 0.0, 0.0};
+    write_frame_row(wv, (size_t)fo, r, I, Trl);
+  }
+  for (int s = 0; s < N; s += nf) {
+    const int k = s + f, n = min(nf, N - s);
+    double m[4] = {0.0, 0.0, 0.0, 0.0};
+    if (k < N) {  // row r of inv(T_k)
+      const double *T = poses + 12 * (size_t)(po + k);
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      double P[12];
-#pragma unroll
-      for (int q = 0; q < 12; ++q) P[q] = __shfl_up_sync(0xffffffffu, M[q], d);
-      if (lane >= d) {
-        double C[12];
-        compose34(P, M, C);
-#pragma unroll
-        for (int q = 0; q < 12; ++q) M[q] = C[q];
-      }
+      for (int j = 0; j < 3; ++j) m[j] = T[4 * j + r];
+      m[3] = -(m[0] * T[3] + m[1] * T[7] + m[2] * T[11]);
     }
-    double G[12];
-    compose34(carry, M, G);
-    if (k < N) write_frame(wv, (size_t)(fo + k + 1), G, Trl);
+    int cur = 0;
 #pragma unroll
-    for (int q = 0; q < 12; ++q) carry[q] = __shfl_sync(0xffffffffu, G[q], 31);
+    for (int j = 0; j < 4; ++j) buf[0][f][4 * r + j] = m[j];
+    __syncthreads();
+    // inclusive scan: M_k <- M_0 M_1 ... M_k (earlier factors on the left)
+    for (int d = 1; d < n; d <<= 1) {
+      if (f >= d) {
+        double p[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p[j] = buf[cur][f - d][4 * r + j];
+        compose_row(p, buf[cur][f], m);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) buf[cur ^ 1][f][4 * r + j] = m[j];
+      cur ^= 1;
+      __syncthreads();
+    }
+    if (s > 0) {
+      double p[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) p[j] = last[4 * r + j];
+      compose_row(p, buf[cur][f], m);
+    }
+    if (k < N) write_frame_row(wv, (size_t)(fo + k + 1), r, m, Trl);
+    __syncthreads();  // (every product with the carried prefix is formed)
+    if (f == nf - 1) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) last[4 * r + j] = m[j];
+    }
+    __syncthreads();
   }
 }
 
@@ -425,7 +459,8 @@ __global__ void __launch_bounds__(32 * kChainWarps) k_chain_df(PlanView pv, Work
 
 int launch_chain(const PlanView &pv, const WorkView &wv, const double *poses, int gate, int f64, void *stream) {
   if (f64)
-    k_chain<<<pv.B, 32, 0, (cudaStream_t)stream>>>(pv, wv, poses, gate);  // one warp (and SM slot) per problem
+    k_chain<<<pv.B, 96 * std::min(kChainFrames / 32, std::max(1, (pv.max_P / 6 + 31) / 32)), 0, (cudaStream_t)stream>>>(
+        pv, wv, poses, gate);
   else
     k_chain_df<<<pv.B, 32 * std::min(kChainWarps, std::max(1, (pv.max_P / 6 + 31) / 32)), 0, (cudaStream_t)stream>>>(
         pv, wv, poses, gate);

@@ -37,10 +37,10 @@ __device__ __forceinline__ T s_entry(const T *A, const T *SL, int P, int r, int 
 // (independent per row) and apply the rank-16 trailing update, the next block's
 // columns first, so that warp 0 factorises the next diagonal block while the other
 // warps update the rest (one block of look-ahead); three barriers per block.
-// Bound by the diagonal blocks' chain in FP32 (one 16-pose window: 35 us with a pivot, its
-// correctly rounded root and reciprocal and fifteen shuffles per column, 29.7 us in groups of
-// four columns) and in FP64 by the FP64 pipe's 2 FMA per cycle and SM (eight solves of a window
-// of up to 16 poses: 613 us with a thread per row, a warp per two columns and a row's columns
+// Bound by the diagonal blocks' chain in FP32 (one 10-pose window: 35 us with a pivot, its
+// correctly rounded root and reciprocal and fifteen shuffles per column, 28.5 us in groups of
+// four columns) and in FP64 by the FP64 pipe's 2 FMA per cycle and SM (eight solves of a 10-pose
+// window: 613 us with a thread per row, a warp per two columns and a row's columns
 // in one lane; 377 us with the work laid out by FP64 instructions as below).  The substitutions are blocked the same way (two barriers per
 // block).  `refine` iterative-refinement steps form the residual g_S - S x
 // (double-float on the FP32 path, FP64 otherwise) from A and S_L in one

@@ -24,18 +24,11 @@ __device__ __forceinline__ constexpr int t6(int i, int j) {  // symmetric 6x6 up
   return i <= j ? i * 6 - (i * (i - 1)) / 2 + (j - i) : j * 6 - (j * (j - 1)) / 2 + (i - j);
 }
 
-// pass A, one thread per (problem, hi):
-// P(i, hi) = sum_{lo <= i} M(lo, hi), each term about its own origin c_lo; the
-// running sum is re-centred from c_{lo-1} to c_lo before adding M(lo, hi), so
-// every partial sum sits at the origin of its row i and only relative centres
-// enter the arithmetic.  Re-centring a record: E_z^T M E_z and E_z^T m for
-// E_z = [[I, 0], [-[z]x, I]] move a record from origin x to origin y = x - z
-// (K^y = K^x E_{x - y}).  With the 6x6 block M = [[P, Q], [Q^T, R]] (upper triangle,
-// 21 values), m = [m_w; m_v] and Z = [z]x:  P' = P - Q Z + Z Q^T - Z R Z,
-// Q' = Q + Z R,  R' = R,  m' = [m_w + Z m_v ; m_v].  Reads and clears the records.
-// The thread holds the whole 27-value running sum, so the shift's shared products
-// are formed once per step (about a sixth of the arithmetic of one lane per
-// component, which matters in FP64):
+// Moving a record from origin x to origin y = x - z: E_z^T M E_z and E_z^T m for
+// E_z = [[I, 0], [-[z]x, I]] (K^y = K^x E_{x - y}).  With the 6x6 block M = [[P, Q], [Q^T, R]]
+// (upper triangle, 21 values), m = [m_w; m_v] and Z = [z]x:  P' = P - Q Z + Z Q^T - Z R Z,
+// Q' = Q + Z R,  R' = R,  m' = [m_w + Z m_v ; m_v].  The thread holds all 27 values, so the
+// shared products are formed once (about a sixth of the arithmetic of one lane per component):
 //   (Z R)[:, j] = z x R[:, j],  (Q Z)[i, :] = -(z x Q[i, :]),  ((Z R) Z)[i, :] = -(z x (Z R)[i, :]),
 //   P' = P - Q Z - (Q Z)^T - (Z R) Z,  Q' = Q + Z R,  m_w' = m_w + z x m_v.
 template <typename V>
@@ -94,36 +87,55 @@ __device__ __forceinline__ void shift_record(V *v, const V *z) {
   v[23] += o[2];
 }
 
-__global__ void __launch_bounds__(64) k_pair_prefix_rec(PlanView pv, WorkView wv) {
+// pass A (FP64), one CTA per (problem, hi): P(i, hi) = sum_{lo <= i} M(lo, hi) about c_i, each
+// M(lo, hi) given about c_lo.  Reads and clears the records.  Every record is moved to the centre
+// of the chain's first frame, the running sums are formed there and each is moved back to its own
+// row's centre: lever arms stay within the frames that saw the pair's landmarks, and the two
+// moves, some 110 FP64 instructions of 64 cycles each, run on all records at once instead of one
+// after the other along the chain (101 poses with windows of 41: 202 us with a thread per chain,
+// 12.7 us so).
+__global__ void __launch_bounds__(SPGO_MAX_WINDOW) k_pair_prefix_rec(PlanView pv, WorkView wv) {
   const int b = blockIdx.y;
   if (!problem_active(wv.lm, b, GATE_RELIN)) return;
-  const int N = pv.p_npose[b], D = pv.p_pair_D[b];
-  const int hi = 1 + blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ double v[SPGO_MAX_WINDOW][27];
+  const int N = pv.p_npose[b], D = pv.p_pair_D[b], hi = 1 + blockIdx.x, tid = threadIdx.x;
   if (hi > N) return;
-  const int fo = pv.p_frame_off[b];
-  double *acc_base = reinterpret_cast<double *>(wv.pair_acc) + (size_t)pv.p_pair_off[b] * 27;
-  double *out_base = reinterpret_cast<double *>(wv.pairF) + (size_t)pv.p_pair_off[b] * 27;
-  const int lo0 = max(0, hi - D);
-  double v[27];
-#pragma unroll
-  for (int k = 0; k < 27; ++k) v[k] = 0.0;
-  for (int lo = lo0; lo < hi; ++lo) {
-    if (lo > lo0) {
-      const Vec3<double> zz = FramesT<double>::rel(wv, fo + lo - 1, 0, fo + lo, 0);
-      const double z[3] = {zz.x, zz.y, zz.z};
-      shift_record(v, z);
-    }
-    double *rec = acc_base + ((size_t)lo * D + (hi - lo - 1)) * 27;
-    double *out = out_base + ((size_t)lo * D + (hi - lo - 1)) * 27;
+  const int fo = pv.p_frame_off[b], lo0 = max(0, hi - D), n = hi - lo0;
+  // record (lo, hi)
+  auto at = [&](int lo) { return ((size_t)pv.p_pair_off[b] + (size_t)lo * D + (hi - lo - 1)) * 27; };
+  auto moved = [&](double *r, int from, int to) {
+    const Vec3<double> zz = FramesT<double>::rel(wv, fo + from, 0, fo + to, 0);
+    const double z[3] = {zz.x, zz.y, zz.z};
+    shift_record(r, z);
+  };
+  for (int q = tid; q < n; q += blockDim.x) {
+    double *rec = reinterpret_cast<double *>(wv.pair_acc) + at(lo0 + q);
     double r[27];
 #pragma unroll
     for (int k = 0; k < 27; ++k) r[k] = rec[k];
 #pragma unroll
-    for (int k = 0; k < 27; ++k) {
-      rec[k] = 0.0;  // cleared for the next linearisation
-      v[k] += r[k];
-      out[k] = v[k];
+    for (int k = 0; k < 27; ++k) rec[k] = 0.0;  // cleared for the next linearisation
+    if (q > 0) moved(r, lo0 + q, lo0);
+#pragma unroll
+    for (int k = 0; k < 27; ++k) v[q][k] = r[k];
+  }
+  __syncthreads();
+  if (tid < 27) {
+    double sum = 0.0;
+    for (int q = 0; q < n; ++q) {
+      sum += v[q][tid];
+      v[q][tid] = sum;
     }
+  }
+  __syncthreads();
+  for (int q = tid; q < n; q += blockDim.x) {
+    double r[27];
+#pragma unroll
+    for (int k = 0; k < 27; ++k) r[k] = v[q][k];
+    if (q > 0) moved(r, lo0, lo0 + q);
+    double *out = reinterpret_cast<double *>(wv.pairF) + at(lo0 + q);
+#pragma unroll
+    for (int k = 0; k < 27; ++k) out[k] = r[k];
   }
 }
 
@@ -157,118 +169,6 @@ __global__ void k_pair_suffix(PlanView pv, WorkView wv) {
   }
 }
 
-template <typename T> struct Pair2;
-template <> struct Pair2<float> {
-  using type = float2;
-  __device__ static float2 make(float a, float b) { return make_float2(a, b); }
-};
-template <> struct Pair2<double> {
-  using type = double2;
-  __device__ static double2 make(double a, double b) { return make_double2(a, b); }
-};
-
-// A(i, j) = Ad_i^T F(i, j) Ad_j about origin c_i: Ad_i = diag(R_i, R_i),
-// Ad_j = [[R_j, 0], [[c_j - c_i]x R_j, R_j]];  g(i) = [R_i^T f_w ; R_i^T f_v].
-// Computed in T, stored as TO (the mixed path reduces in FP64 and stores FP32: one
-// rounding of the exact sums)
-template <typename T, typename TO = T>
-__global__ void k_pairs_to_A(PlanView pv, WorkView wv) {
-  const int b = blockIdx.y;
-  if (!problem_active(wv.lm, b, GATE_RELIN)) return;
-  const int N = pv.p_npose[b], D = pv.p_pair_D[b];
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= N * D) return;
-  const int i = t / D, e = t % D;
-  if (e >= min(D, N - i)) return;
-  const int j = i + e;
-  const int P = 6 * N;
-  const int fo = pv.p_frame_off[b];
-  // the record and both rotations in registers first (the A stores below could
-  // otherwise alias them and force reloads)
-  const T *Fg = reinterpret_cast<const T *>(wv.pairF) + ((size_t)pv.p_pair_off[b] + (size_t)i * D + e) * 27;
-  const T *Rig = FramesT<T>::R(wv, fo + i, 0);
-  const T *Rjg = FramesT<T>::R(wv, fo + j, 0);
-  T F[27], Ri[9], Rj[9];
-#pragma unroll
-  for (int k = 0; k < 27; ++k) F[k] = Fg[k];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    Ri[k] = Rig[k];
-    Rj[k] = Rjg[k];
-  }
-  const Vec3<T> cji = FramesT<T>::rel(wv, fo + j, 0, fo + i, 0);
-  // C R_j with C = [c_j - c_i]x
-  T CRj[9];
-  {
-    const T X[9] = {T(0), -cji.z, cji.y, cji.z, T(0), -cji.x, -cji.y, cji.x, T(0)};
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        CRj[3 * r + c] = X[3 * r] * Rj[c] + X[3 * r + 1] * Rj[3 + c] + X[3 * r + 2] * Rj[6 + c];
-  }
-  // the whole 6x6 block first: out[r][c] = A(6i + r, 6j + c)
-  T out[6][6];
-#pragma unroll
-  for (int col = 0; col < 6; ++col) {
-    T adj[6];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      adj[r] = col < 3 ? Rj[3 * r + col] : T(0);
-      adj[3 + r] = col < 3 ? CRj[3 * r + col] : Rj[3 * r + col - 3];
-    }
-    T w[6];
-#pragma unroll
-    for (int r = 0; r < 6; ++r) {
-      T a = T(0);
-#pragma unroll
-      for (int k = 0; k < 6; ++k) a += F[t6(r, k)] * adj[k];
-      w[r] = a;
-    }
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      out[r][col] = Ri[r] * w[0] + Ri[3 + r] * w[1] + Ri[6 + r] * w[2];
-      out[3 + r][col] = Ri[r] * w[3] + Ri[3 + r] * w[4] + Ri[6 + r] * w[5];
-    }
-  }
-  // both copies as pairs of adjacent elements (every offset below is even and the
-  // workspace segment 256-byte aligned): the block (i, j) row by row, and for
-  // i != j its transpose (j, i), whose rows are 6 elements at 6i of rows 6j + c
-  using V2 = typename Pair2<TO>::type;
-  TO *A = reinterpret_cast<TO *>(wv.A) + pv.p_S_off[b];
-#pragma unroll
-  for (int r = 0; r < 6; ++r)
-#pragma unroll
-    for (int c = 0; c < 6; c += 2)
-      *reinterpret_cast<V2 *>(A + (size_t)(6 * i + r) * P + 6 * j + c) =
-          Pair2<TO>::make((TO)out[r][c], (TO)out[r][c + 1]);
-  if (i != j) {
-#pragma unroll
-    for (int c = 0; c < 6; ++c)
-#pragma unroll
-      for (int r = 0; r < 6; r += 2)
-        *reinterpret_cast<V2 *>(A + (size_t)(6 * j + c) * P + 6 * i + r) =
-            Pair2<TO>::make((TO)out[r][c], (TO)out[r + 1][c]);
-  }
-  if (e == 0) {
-    const T *f = F + 21;
-    TO *g = reinterpret_cast<TO *>(wv.g) + pv.p_param_off[b] + 6 * i;
-    T gi[6];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      gi[r] = Ri[r] * f[0] + Ri[3 + r] * f[1] + Ri[6 + r] * f[2];
-      gi[3 + r] = Ri[r] * f[3] + Ri[3 + r] * f[4] + Ri[6 + r] * f[5];
-    }
-#pragma unroll
-    for (int r = 0; r < 6; ++r) g[r] = (TO)gi[r];
-    if (wv.gacc) {  // the mixed path's refined step: the gradient unrounded, for its predicted decrease
-      double *ga = wv.gacc + pv.p_param_off[b] + 6 * i;
-#pragma unroll
-      for (int r = 0; r < 6; ++r) ga[r] = (double)gi[r];
-    }
-  }
-}
-
 // ---- the mixed path's pair reduction, in double-float ----------------------------
 // The records arrive as FP64 sums (the linearisation's atomics).  FP64 arithmetic runs at
 // a small fraction of the FP32 rate on this GPU, so the reduction runs in double-float
@@ -276,7 +176,7 @@ __global__ void k_pairs_to_A(PlanView pv, WorkView wv) {
 // of re-centring a running sum along each chain (a serial chain of shifts), every record
 // is moved once to the problem's own origin o = c_0 (its lever arms are at most the
 // window's extent, tens of metres, which costs a few of the 48 bits), the prefix and
-// suffix sums run about o, and each block moves its sum from o to c_i on the way to A.
+// suffix sums run about o, and A and g are formed from the sums about o.
 __device__ __forceinline__ void df_rel_c(const WorkView &wv, int fx, int fy, df *z) {  // c_x - c_y, left cameras
 #pragma unroll
   for (int k = 0; k < 3; ++k)
@@ -366,95 +266,104 @@ __global__ void __launch_bounds__(kPrThreads) k_pair_scan_df(PlanView pv, WorkVi
   }
 }
 
-// A(i, j) = Ad_i^T F(i, j) Ad_j about c_i (F moved there from o first) and g(i), in
-// double-float, rounded once to FP32; the unrounded g also to gacc (the refined step's
-// predicted decrease)
-__global__ void __launch_bounds__(128) k_pairs_to_A_df(PlanView pv, WorkView wv) {
+// A(i, j) = Ad_i^T F(i, j) Ad_j and g(i) = the same of F's gradient, F about an origin o (FP64:
+// c_i; mixed: the problem's c_0) and Ad_k = [[R_k, 0], [[c_k - o]x R_k, R_k]]; the mixed path in
+// double-float, rounded once to FP32, the unrounded g also to gacc (the refined step's predicted
+// decrease).  One thread per column of a block: some 70 multiply-adds in a chain-bound kernel,
+// where a thread per block had 350 (FP64, 64 cycles each: 10 us a window), and 460 with the move
+// of F from o to c_i that the mixed path made first (16.6 us a window; 5.2 us so).
+template <typename T>
+__global__ void __launch_bounds__(128) k_pairs_to_A(PlanView pv, WorkView wv) {
+  constexpr bool f64 = std::is_same<T, double>::value;
+  using V = typename std::conditional<f64, double, df>::type;
   const int b = blockIdx.y;
   if (!problem_active(wv.lm, b, GATE_RELIN)) return;
   const int N = pv.p_npose[b], D = pv.p_pair_D[b];
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= N * D) return;
-  const int i = t / D, e = t % D;
-  if (e >= min(D, N - i)) return;
-  const int j = i + e;
-  const int P = 6 * N;
-  const int fo = pv.p_frame_off[b];
-  const df *Fg = reinterpret_cast<const df *>(wv.pairF) + ((size_t)pv.p_pair_off[b] + (size_t)i * D + e) * 27;
-  df F[27], Ri[9], Rj[9];
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, col = t % 6, i = t / (6 * D), e = t / 6 - i * D;
+  if (i >= N || e >= min(D, N - i)) return;
+  const int j = i + e, P = 6 * N, fo = pv.p_frame_off[b], cc = col < 3 ? col : col - 3;
+  const V *Fg = reinterpret_cast<const V *>(wv.pairF) + ((size_t)pv.p_pair_off[b] + (size_t)i * D + e) * 27;
+  V F[21], Ri[9], a[3], lj[3], li[3];  // a: column cc of R_j
 #pragma unroll
-  for (int k = 0; k < 27; ++k) F[k] = Fg[k];
-  {
+  for (int k = 0; k < 21; ++k) F[k] = Fg[k];
+  if constexpr (f64) {
+    const double *ri = FramesT<double>::R(wv, fo + i, 0), *rj = FramesT<double>::R(wv, fo + j, 0);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Ri[k] = ri[k];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) a[k] = rj[3 * k + cc];
+    const Vec3<double> c = FramesT<double>::rel(wv, fo + j, 0, fo + i, 0);
+    lj[0] = c.x, lj[1] = c.y, lj[2] = c.z;
+  } else {
     const float *h = wv.fr_Rf + (size_t)(fo + i) * 18, *l = wv.fr_Rl + (size_t)(fo + i) * 18;
-    const float *hj = wv.fr_Rf + (size_t)(fo + j) * 18, *lj = wv.fr_Rl + (size_t)(fo + j) * 18;
+    const float *hj = wv.fr_Rf + (size_t)(fo + j) * 18, *ljp = wv.fr_Rl + (size_t)(fo + j) * 18;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      Ri[k] = df{h[k], l[k]};
-      Rj[k] = df{hj[k], lj[k]};
+    for (int k = 0; k < 9; ++k) Ri[k] = df{h[k], l[k]};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) a[k] = df{hj[3 * k + cc], ljp[3 * k + cc]};
+    df_rel_c(wv, fo + j, fo, lj);
+    df_rel_c(wv, fo + i, fo, li);
+  }
+  // column col of Ad_j: [a; l_j x a] (col < 3), [0; a]
+  V ad[6];
+  cross3(lj, a, ad + 3);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    ad[k] = col < 3 ? a[k] : V{};
+    ad[3 + k] = col < 3 ? ad[3 + k] : a[k];
+  }
+  V w[6];
+#pragma unroll
+  for (int r = 0; r < 6; ++r) {
+    V u = F[t6(r, 0)] * ad[0];
+#pragma unroll
+    for (int k = 1; k < 6; ++k) u = u + F[t6(r, k)] * ad[k];
+    w[r] = u;
+  }
+  auto to_frame_i = [&](V *x) {  // x[0..2] -= l_i x x[3..5]
+    if constexpr (!f64) {
+      V o[3];
+      cross3(li, x + 3, o);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) x[k] = x[k] - o[k];
     }
-  }
-  if (i > 0) {
-    df z[3];
-    df_rel_c(wv, fo, fo + i, z);  // from o = c_0 to c_i
-    shift_record(F, z);
-  }
-  df cji[3];
-  df_rel_c(wv, fo + j, fo + i, cji);
-  // C R_j with C = [c_j - c_i]x
-  df CRj[9];
+  };
+  auto round_t = [](const V &x) {
+    if constexpr (f64)
+      return x;
+    else
+      return df_to_float(x);
+  };
+  to_frame_i(w);
+  T out[6];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    CRj[c] = cji[1] * Rj[6 + c] - cji[2] * Rj[3 + c];
-    CRj[3 + c] = cji[2] * Rj[c] - cji[0] * Rj[6 + c];
-    CRj[6 + c] = cji[0] * Rj[3 + c] - cji[1] * Rj[c];
+  for (int r = 0; r < 3; ++r) {
+    out[r] = round_t(Ri[r] * w[0] + Ri[3 + r] * w[1] + Ri[6 + r] * w[2]);
+    out[3 + r] = round_t(Ri[r] * w[3] + Ri[3 + r] * w[4] + Ri[6 + r] * w[5]);
   }
-  float out[6][6];
+  T *A = reinterpret_cast<T *>(wv.A) + pv.p_S_off[b];
 #pragma unroll
-  for (int col = 0; col < 6; ++col) {
-    // column col of Ad_j: [R_j e_col ; C R_j e_col] (col < 3), [0 ; R_j e_(col-3)]
-    df w[6];
+  for (int r = 0; r < 6; ++r) A[(size_t)(6 * i + r) * P + 6 * j + col] = out[r];
+  if (i != j) {  // its transpose: 6 elements at 6i of row 6j + col (even offsets in a 256-byte aligned segment)
+    using T2 = typename std::conditional<f64, double2, float2>::type;
+    T2 *dst = reinterpret_cast<T2 *>(A + (size_t)(6 * j + col) * P + 6 * i);
 #pragma unroll
-    for (int r = 0; r < 6; ++r) {
-      df a = col < 3 ? F[t6(r, 0)] * Rj[col] + F[t6(r, 1)] * Rj[3 + col] + F[t6(r, 2)] * Rj[6 + col]
-                     : df_make(0.f);
-      const int cc = col < 3 ? col : col - 3;
-      const df *ad = col < 3 ? CRj : Rj;
-      a = a + F[t6(r, 3)] * ad[cc] + F[t6(r, 4)] * ad[3 + cc] + F[t6(r, 5)] * ad[6 + cc];
-      w[r] = a;
+    for (int r = 0; r < 3; ++r) dst[r] = T2{out[2 * r], out[2 * r + 1]};
+  } else {
+    V f[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) f[k] = Fg[21 + k];
+    to_frame_i(f);
+    V gr{};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {  // (Ri in registers: its column by selection)
+      const V rk = cc == 0 ? Ri[3 * k] : cc == 1 ? Ri[3 * k + 1] : Ri[3 * k + 2];
+      gr = gr + rk * (col < 3 ? f[k] : f[3 + k]);
     }
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      out[r][col] = df_to_float(Ri[r] * w[0] + Ri[3 + r] * w[1] + Ri[6 + r] * w[2]);
-      out[3 + r][col] = df_to_float(Ri[r] * w[3] + Ri[3 + r] * w[4] + Ri[6 + r] * w[5]);
-    }
-  }
-  float *A = reinterpret_cast<float *>(wv.A) + pv.p_S_off[b];
-#pragma unroll
-  for (int r = 0; r < 6; ++r)
-#pragma unroll
-    for (int c = 0; c < 6; c += 2)
-      *reinterpret_cast<float2 *>(A + (size_t)(6 * i + r) * P + 6 * j + c) = make_float2(out[r][c], out[r][c + 1]);
-  if (i != j) {
-#pragma unroll
-    for (int c = 0; c < 6; ++c)
-#pragma unroll
-      for (int r = 0; r < 6; r += 2)
-        *reinterpret_cast<float2 *>(A + (size_t)(6 * j + c) * P + 6 * i + r) = make_float2(out[r][c], out[r + 1][c]);
-  }
-  if (e == 0) {
-    const df *f = F + 21;
-    float *g = reinterpret_cast<float *>(wv.g) + pv.p_param_off[b] + 6 * i;
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      const df gw = Ri[r] * f[0] + Ri[3 + r] * f[1] + Ri[6 + r] * f[2];
-      const df gv = Ri[r] * f[3] + Ri[3 + r] * f[4] + Ri[6 + r] * f[5];
-      g[r] = df_to_float(gw);
-      g[3 + r] = df_to_float(gv);
-      if (wv.gacc) {
-        wv.gacc[pv.p_param_off[b] + 6 * i + r] = df_to_double(gw);
-        wv.gacc[pv.p_param_off[b] + 6 * i + 3 + r] = df_to_double(gv);
-      }
-    }
+    const int row = pv.p_param_off[b] + 6 * i + col;
+    reinterpret_cast<T *>(wv.g)[row] = round_t(gr);
+    if constexpr (!f64)
+      if (wv.gacc) wv.gacc[row] = df_to_double(gr);
   }
 }
 
@@ -477,12 +386,12 @@ int launch_system(const PlanView &pv, const WorkView &wv, int gate, void *stream
       k_pair_scan_df<2><<<grid, 128, 0, st>>>(pv, wv);
       ++g_launches;
     }
-    k_pairs_to_A_df<<<dim3(grid_for((long long)nmax * nd, 128), pv.B), 128, 0, st>>>(pv, wv);
+    k_pairs_to_A<float><<<dim3(grid_for((long long)nmax * nd * 6, 128), pv.B), 128, 0, st>>>(pv, wv);
     g_launches += 3;
   } else {
-    k_pair_prefix_rec<<<dim3(grid_for(nmax, 64), pv.B), 64, 0, st>>>(pv, wv);
+    k_pair_prefix_rec<<<dim3(nmax, pv.B), 32 * grid_for(std::min(nd, nmax), 32), 0, st>>>(pv, wv);
     k_pair_suffix<double><<<dim3(grid_for((long long)nmax * 27, 128), pv.B), 128, 0, st>>>(pv, wv);
-    k_pairs_to_A<double, T><<<dim3(grid_for((long long)nmax * nd, 128), pv.B), 128, 0, st>>>(pv, wv);
+    k_pairs_to_A<double><<<dim3(grid_for((long long)nmax * nd * 6, 128), pv.B), 128, 0, st>>>(pv, wv);
     g_launches += 3;
   }
   return (int)cudaGetLastError();

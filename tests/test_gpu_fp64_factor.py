@@ -2,7 +2,8 @@
 their shapes: one CTA with the packed factor (16-wide blocks: one narrow block, an exact
 multiple, every kind of remainder, the largest number of rows left), and 32-column panels
 spread over CTAs (an exact multiple, narrow last panels, bands below one panel, below the
-substitutions' 64-row blocks, and as wide as the matrix).  One damped step near the optimum;
+substitutions' 64-row blocks, and as wide as the matrix); the last three also at the edges of
+the pose chain's passes of 128 frames.  One damped step near the optimum;
 tolerance 1e-8 of the step, the one the FP64 GN steps are held to elsewhere."""
 import numpy as np
 import pytest
@@ -15,7 +16,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n_poses,window", [(1, 2), (2, 2), (3, 3), (8, 4), (11, 6), (16, 8), (21, 9), (27, 27), (34, 12),
-                                            (38, 2), (43, 4), (48, 6), (53, 11), (58, 16), (64, 44), (41, 41)])
+                                            (38, 2), (43, 4), (48, 6), (53, 11), (58, 16), (64, 44), (41, 41),
+                                            (128, 3), (129, 5), (300, 2)])
 def test_fp64_step_matches_dense_solve(built_lib, cuda_device, n_poses, window):
     p = corridor(700 + n_poses, n_poses, window)
     p.poses, p.alpha = p.gt_poses.copy(), p.gt_alpha.copy()
