@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(32 * kLgPanelRows) k_lg_panel(PlanView pv, Wor
     if (warp == k % W) ck[lane] = a[k / W];
     __syncthreads();
     const double d = ck[k];
-    bad = bad || !(d > 0.0) || !(d < INFINITY);
+    bad = bad || !pivot_ok(d);
     const double t = ck[lane] * rcp_pivot(d);  // rows above k: values nobody reads
     if (warp == k % W) {
       U[k][lane] = t;

@@ -476,26 +476,22 @@ int launch_resid_pass(const PlanView &pv, const WorkView &wv, const Params &prm,
 // component), no atomics.
 constexpr int kRsThreads = 256;
 
-// shared memory: centres, row and column sums | cb | y | tmp | the packed factor
-// followed by its pivots' reciprocals (as stored by the factorisation)
-__host__ __device__ inline size_t rs_layout(int max_Ps, int max_N, size_t *off_cb, size_t *off_y, size_t *off_tmp,
-                                            size_t *off_L) {
+// shared memory: centres, row and column sums | cb | y | the packed factor
+// (as stored by the factorisation)
+__host__ __device__ inline size_t rs_layout(int max_Ps, int max_N, size_t *off_cb, size_t *off_y, size_t *off_L) {
   auto up = [](size_t x) { return (x + 15) & ~(size_t)15; };
   size_t o = up((size_t)(max_N + 1) * 15 * sizeof(double));  // centres [N+1][3], rows, columns [N+1][6]
   *off_cb = o;
   o = up(o + (size_t)max_Ps * sizeof(int));
   *off_y = o;
   o = up(o + (size_t)max_Ps * sizeof(float));
-  *off_tmp = o;
-  o = up(o + (size_t)kPanel * sizeof(float));
   *off_L = o;
-  o = up(o + ((size_t)max_Ps * (max_Ps + 1) / 2 + max_Ps) * sizeof(float));
-  return o;
+  return up(o + ((size_t)max_Ps * (max_Ps + 1) / 2 + kPanel) * sizeof(float));  // (+ kPanel: chol_substitute)
 }
 
 size_t resid_solve_smem(int max_P_small, int max_N) {
-  size_t a, b, c, d;
-  return rs_layout(max_P_small, max_N, &a, &b, &c, &d);
+  size_t a, b, c;
+  return rs_layout(max_P_small, max_N, &a, &b, &c);
 }
 
 // 16-byte asynchronous global -> shared copies (no registers held while in flight)
@@ -514,17 +510,17 @@ __global__ void __launch_bounds__(kRsThreads) k_resid_solve(PlanView pv, WorkVie
   const int N = pv.p_npose[b], D = pv.p_pair_D[b], P = 6 * N;
   const int fo = pv.p_frame_off[b], po = pv.p_param_off[b];
   const int tid = threadIdx.x, nt = blockDim.x;
-  size_t o_cb, o_y, o_tmp, o_L;
-  rs_layout(pv.max_P_small, pv.max_P / 6, &o_cb, &o_y, &o_tmp, &o_L);
+  size_t o_cb, o_y, o_L;
+  rs_layout(pv.max_P_small, pv.max_P / 6, &o_cb, &o_y, &o_L);
   const bool small = P <= pv.max_P_small;
   if (!small && wv.lg_red) return;  // wide problems: the grid-wide kernels below
   const size_t npk = (size_t)P * (P + 1) / 2;
   float *Lm = reinterpret_cast<float *>(smem_raw + o_L);
   if (small) {
-    // the stored factor and pivots (contiguous, 16-byte aligned: S offsets are multiples
+    // the stored factor (contiguous, 16-byte aligned: S offsets are multiples
     // of 36 floats) start copying now and land while the pair duals are reduced
     const float *fac = wv.facs + pv.p_S_off[b];
-    const size_t n = npk + P, n4 = n / 4;
+    const size_t n = npk, n4 = n / 4;
     for (size_t k = tid; k < n4; k += nt) cp_async16(Lm + 4 * k, fac + 4 * k);
     for (size_t k = 4 * n4 + tid; k < n; k += nt) Lm[k] = fac[k];
   }
@@ -607,12 +603,10 @@ __global__ void __launch_bounds__(kRsThreads) k_resid_solve(PlanView pv, WorkVie
   }
   if (!small) return;  // the multi-CTA substitutions (k_chol_large.cu) follow
   int *cb = reinterpret_cast<int *>(smem_raw + o_cb);
-  float *tmp = reinterpret_cast<float *>(smem_raw + o_tmp);
-  const float *dinv = Lm + npk;
   for (int k = tid; k < P; k += nt) cb[k] = k * P - (k * (k + 1)) / 2;
   cp_async_wait_all();
   __syncthreads();
-  chol_substitute<float>(Lm, cb, y, dinv, tmp, P);
+  chol_substitute<float>(Lm, cb, y, nullptr, P);
   __shared__ unsigned mx_dx, mx_x;  // largest |correction|, |step| (float bits: non-negative floats order as ints)
   if (tid == 0) mx_dx = mx_x = 0u;
   __syncthreads();

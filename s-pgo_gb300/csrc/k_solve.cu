@@ -31,22 +31,40 @@ __device__ __forceinline__ T s_entry(const T *A, const T *SL, int P, int r, int 
   return v;
 }
 
-// One CTA per problem: assemble S (lower) into the factor storage, then a
-// right-looking blocked Cholesky S = L L^T with 16-column blocks: warp 0
-// factorises the 16x16 diagonal block, all threads solve the rows below it
-// (independent per row) and apply the rank-16 trailing update, the next block's
-// columns first, so that warp 0 factorises the next diagonal block while the other
-// warps update the rest (one block of look-ahead); three barriers per block.
-// Bound by the diagonal blocks' chain in FP32 (one 10-pose window: 35 us with a pivot, its
-// correctly rounded root and reciprocal and fifteen shuffles per column, 28.5 us in groups of
-// four columns) and in FP64 by the FP64 pipe's 2 FMA per cycle and SM (eight solves of a 10-pose
-// window: 613 us with a thread per row, a warp per two columns and a row's columns
-// in one lane; 377 us with the work laid out by FP64 instructions as below).  The substitutions are blocked the same way (two barriers per
-// block).  `refine` iterative-refinement steps form the residual g_S - S x
-// (double-float on the FP32 path, FP64 otherwise) from A and S_L in one
-// coalesced pass over the lower triangle.  Clears the S_L / g_L tiles it consumed.
+// FP64: a diagonal block takes 10.7k cycles alone and up to 18k beside a warp of updates; elements
+// (1150 cycles of a quarter SM per 32) beyond which the update lasts longer than that anyway.
+constexpr int kDrawAll = 1700;
+
+// element o of the n of a packed lower triangle that ends at (P - 1, P - 1), if its row is at
+// least r0
+template <typename F>
+__device__ __forceinline__ void element(int P, int n, int o, int r0, F &&f) {
+  const int r = n - 1 - o;  // from the end: column P - 1 - jj holds jj + 1 elements
+  float root;  // (to a few ulp: the next lines settle it)
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(root) : "f"(8.f * (float)r + 1.f));
+  int jj = (int)((root - 1.f) * 0.5f);
+  jj += (jj + 1) * (jj + 2) / 2 <= r;
+  jj -= jj * (jj + 1) / 2 > r;
+  const int i = P - 1 - (r - jj * (jj + 1) / 2);
+  if (i >= r0) f(i, P - 1 - jj);
+}
+
+// One CTA per problem: assemble S (lower) into the factor storage, then a right-looking blocked
+// Cholesky S = L L^T with 16-column blocks: warp 0 factorises the 16x16 diagonal block, all
+// threads solve the rows below it (independent per row) and apply the rank-16 update, the next
+// diagonal block first, so that warp 0 factorises it while the other warps update the rest (one
+// block of look-ahead); three barriers per block.
+// Bound by the diagonal blocks' chain and the barriers in FP32 (one 10-pose window: 35 us with a
+// pivot, its root, its reciprocal and fifteen shuffles per column, the factor's columns found
+// through a table and two barriers per block of the substitutions; 18.4 us so; 64 windows of up to
+// 32 poses: 115 and 83 us) and in FP64 by the FP64 pipe's 2 FMA per cycle and SM (eight solves of
+// a 10-pose window: 613 us with a thread per row, a warp per two columns and a row's columns in
+// one lane; 300 us laid out by FP64 instructions as below).
+// `refine` iterative-refinement steps form the residual g_S - S x (double-float on the FP32 path,
+// FP64 otherwise) from A and S_L in one coalesced pass over the lower triangle.  Clears the
+// S_L / g_L tiles it consumed.
 template <typename T>
-__device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *xs, T *dinv, T *tmp, T *colacc,
+__device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *xs, T *dinv, T *colacc,
                                   const T *A, T *SL, const T *g, T *gL, double lam, int P, int refine,
                                   int *fail_s) {
 #define ix(i, j) (cb[(j)] + (i))
@@ -92,25 +110,32 @@ __device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *
   if (tid == 0) *fail_s = 0;
   __shared__ int drawn;  // FP64: elements of the trailing update handed out
   __syncthreads();
-  // warp 0: the diagonal block [kb, kb + kPanel) in registers; lane i < w holds row i
-  // (a[j] = L(kb+i, kb+j), j <= i; rows past the last block's w are the identity's).
-  // FP32: four columns at a time, their 4x4 pivot block factored by every lane from ten
-  // shuffles, its rows then exchanged through shared memory, so that the chain holds one
-  // exchange per four columns.  FP64, where one instruction of the warp takes 64 cycles: lane
-  // (i, h) holds row i's columns of parity h, and a column costs three for 1 / d, one for its
-  // column of the unit factor U = a / d and one per two later columns; 1 / sqrt(d) for all
-  // columns at once at the end (133 instructions a block; 330 with a row's 16 columns in a lane
-  // and the library's square root and reciprocal).  The block keeps U, for the row solves and
-  // the substitutions.
+  // warp 0: the diagonal block [kb, kb + kPanel) in registers (rows past the last block's w are
+  // the identity's).
+  // FP32: lane i holds row i.  Four columns at a time, their 4x4 pivot block factored by every
+  // lane from ten shuffles, its rows then exchanged through shared memory, so that the chain
+  // holds one exchange per four columns.  The factor goes to Ld (column-major, for the row solves
+  // and the inversion), 1 / L(k, k) to ri.
+  // FP64, where one instruction of the warp takes 64 cycles: lane (i, h) holds row i's columns of
+  // parity h, and a column costs four for its column t = a / d of the unit factor U (from the FP32
+  // estimate y of 1 / d: e = 1 - d y, t = (a y) (1 + e + e^2)) and one per two later columns;
+  // 1 / sqrt(d) for all columns at once at the end.  The next pivot's estimate starts before the
+  // other columns' updates.  The block keeps U, for the row solves and the substitutions.  A
+  // pivot out of the estimate's range sends the block through the library's reciprocal.
+  constexpr bool kF64 = std::is_same<T, double>::value;
+  auto col = [&](int kb, int c) { return c * (P - kb) - c * (c + 1) / 2; };  // cb[kb + c] - cb[kb]
+  __shared__ __align__(16) T Ld[2][kF64 ? 4 : kPanel * kPanel];
+  __shared__ __align__(16) T ri[2][kF64 ? 4 : kPanel];
   auto factor_diag = [&](int kb) {
     const int w = min(kb + kPanel, P) - kb;
     bool bad = false;
-    if constexpr (std::is_same<T, float>::value) {
+    if constexpr (!kF64) {
+      __shared__ __align__(16) float rows[2][4 * kPanel];
+      float *dst = Ld[(kb / kPanel) & 1], *rdst = ri[(kb / kPanel) & 1];
       float a[kPanel];
 #pragma unroll
       for (int j = 0; j < kPanel; ++j)
         a[j] = (lane < w && j <= lane) ? Lm[ix(kb + lane, kb + j)] : (lane == j ? 1.f : 0.f);
-      __shared__ __align__(16) float rows[2][4 * kPanel];
       auto rsq = [&](float d) {  // NaN unless 0 < d < inf
         float r = rsqrtf(d);
         r = fmaf(0.5f * r, fmaf(-d * r, r, 1.f), r);
@@ -136,7 +161,11 @@ __device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *
         a[k + 1] = fmaf(-a[k], l10, a[k + 1]) * r1;
         a[k + 2] = fmaf(-a[k + 1], l21, fmaf(-a[k], l20, a[k + 2])) * r2;
         a[k + 3] = fmaf(-a[k + 2], l32, fmaf(-a[k + 1], l31, fmaf(-a[k], l30, a[k + 3]))) * r3;
-        if (lane < 4 && k + lane < w) dinv[kb + k + lane] = lane == 0 ? r0 : lane == 1 ? r1 : lane == 2 ? r2 : r3;
+        if (lane == 0) *reinterpret_cast<float4 *>(rdst + k) = make_float4(r0, r1, r2, r3);
+        if (lane < kPanel) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) dst[(k + q) * kPanel + lane] = a[k + q];
+        }
         if (k + 4 < kPanel) {
           float *xk = rows[(k >> 2) & 1];  // (double-buffered: one warp barrier per four columns)
           if (lane < kPanel)
@@ -149,53 +178,101 @@ __device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *
           }
         }
       }
-#pragma unroll
-      for (int j = 0; j < kPanel; ++j)
-        if (lane < w && j <= lane) Lm[ix(kb + lane, kb + j)] = a[j];
     } else {
       const int i = lane & 15, h = lane >> 4;
-      double a[kPanel / 2], dk = 1.0;
+      double a[kPanel / 2], t[kPanel], dk = 1.0;
 #pragma unroll
       for (int c = 0; c < kPanel / 2; ++c) {
         const int j = 2 * c + h;
         a[c] = (i < w && j <= i) ? Lm[ix(kb + i, kb + j)] : (i == j ? 1.0 : 0.0);
       }
+      bool odd = false;
+      double d = __shfl_sync(0xffffffffu, a[0], 0);
 #pragma unroll
       for (int k = 0; k < kPanel; ++k) {
         const int from = 16 * (k & 1);  // the half that holds column k
-        const double d = __shfl_sync(0xffffffffu, a[k / 2], k + from);
-        bad = bad || !(d > 0.0) || !(d < INFINITY);
+        bad |= !pivot_ok(d);
+        odd |= !pivot_in_range(d);
         if (lane == k) dk = d;
-        const double t = __shfl_sync(0xffffffffu, a[k / 2], i + from) * rcp_pivot(d);
-        if (h == 0 && i > k && i < w) Lm[ix(kb + i, kb + k)] = t;
+        const double y = rcp_estimate(d), e = fma(-d, y, 1.0), e2 = fma(e, e, e);
+        const double u = __shfl_sync(0xffffffffu, a[k / 2], i + from) * y;
+        t[k] = fma(u, e2, u);
+        double ajk[kPanel / 2];
 #pragma unroll
-        for (int c = (k + 1) / 2; c < kPanel / 2; ++c) {
-          const double ajk = __shfl_sync(0xffffffffu, a[k / 2], 2 * c + h + from);
-          if (2 * c + h > k) a[c] = fma(-t, ajk, a[c]);  // (rows above k: values nobody reads)
+        for (int c = (k + 1) / 2; c < kPanel / 2; ++c) ajk[c] = __shfl_sync(0xffffffffu, a[k / 2], 2 * c + h + from);
+#pragma unroll
+        for (int c = (k + 1) / 2; c < kPanel / 2; ++c) {  // (rows above k: values nobody reads)
+          if (2 * c + h > k) a[c] = fma(-t[k], ajk[c], a[c]);
+          if (c == (k + 1) / 2) d = __shfl_sync(0xffffffffu, a[c], k + 1 + 16 * ((k + 1) & 1));
         }
+      }
+      if (odd) {  // (what followed the pivot out of range above is void)
+        bad = false;
+        for (int k = 0; k < w; ++k) {  // lane = row, on the block in shared memory
+          const double dd = Lm[ix(kb + k, kb + k)], tk = lane > k && lane < w ? Lm[ix(kb + lane, kb + k)] / dd : 0.0;
+          bad = bad || !pivot_ok(dd);
+          if (lane == k) dk = dd;
+          for (int j = k + 1; j < w; ++j)
+            if (lane >= j && lane < w) Lm[ix(kb + lane, kb + j)] -= tk * Lm[ix(kb + j, kb + k)];
+          __syncwarp();
+          if (lane > k && lane < w) Lm[ix(kb + lane, kb + k)] = tk;
+          __syncwarp();
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < kPanel; ++k)
+          if (h == 0 && i > k && i < w) Lm[ix(kb + i, kb + k)] = t[k];
       }
       const double y = rsqrt_pivot(dk);  // lane = column
       if (lane < w) dinv[kb + lane] = y;
     }
     if (bad && lane == 0) *fail_s = 1;
   };
-  // the update of columns [c0, c1) (rows i >= j) with the finished block kb: warp wi of
-  // nwu, KC columns per warp pass (each loaded panel row serves KC columns)
-  auto update_cols = [&](auto kc_tag, const int (&cbk)[kPanel], int w, int c0, int c1, int wi, int nwu) {
-    constexpr int KC = decltype(kc_tag)::value;
-    for (int j0 = c0 + KC * wi; j0 < c1; j0 += KC * nwu) {
+  // FP32, one warp: the inverse of a finished diagonal block to its place, lane = column
+  auto invert_diag = [&](int kb) {
+    if constexpr (!kF64) {
+      const int w = min(kb + kPanel, P) - kb;
+      const float *src = Ld[(kb / kPanel) & 1], *r = ri[(kb / kPanel) & 1];
+      float v[kPanel];
+#pragma unroll
+      for (int k = 0; k < kPanel; ++k) v[k] = k == lane ? 1.f : 0.f;
+#pragma unroll
+      for (int k = 0; k < kPanel; ++k) {
+        v[k] *= r[k];
+#pragma unroll
+        for (int q = (k + 1) / 4; q < kPanel / 4; ++q) {
+          const float4 l = *reinterpret_cast<const float4 *>(src + k * kPanel + 4 * q);
+          const float lv[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+          for (int m = 0; m < 4; ++m)
+            if (4 * q + m > k) v[4 * q + m] = fmaf(-v[k], lv[m], v[4 * q + m]);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < kPanel; ++k)
+        if (lane <= k && k < w) Lm[ix(kb + k, kb + lane)] = v[k];
+    }
+  };
+  // FP32: the update of columns [c0, P), rows from max(j, r0), with the finished block kb: warp wi
+  // of nwu, four columns per warp pass (each loaded panel row serves four columns; an element per
+  // thread, which reads eight times as much of the panel, cost 64 windows of up to 32 poses 5 % and
+  // gained a 10-pose window nothing)
+  auto update_cols = [&](int kb, int c0, int r0, int wi, int nwu) {
+    const T *pan = Lm + cb[kb];
+    constexpr int KC = 4;
+    for (int j0 = c0 + KC * wi; j0 < P; j0 += KC * nwu) {
       T ljk[KC][kPanel];
 #pragma unroll
       for (int c = 0; c < KC; ++c)
 #pragma unroll
-        for (int k = 0; k < kPanel; ++k) ljk[c][k] = (k < w && j0 + c < c1) ? Lm[cbk[k] + j0 + c] : T(0);
-      for (int i = j0 + lane; i < P; i += 32) {
+        for (int k = 0; k < kPanel; ++k) ljk[c][k] = pan[col(kb, k) + min(j0 + c, P - 1)];
+      for (int i = max(j0, r0) + lane; i < P; i += 32) {
         T li[kPanel];
 #pragma unroll
-        for (int k = 0; k < kPanel; ++k) li[k] = Lm[cbk[k] + i];
+        for (int k = 0; k < kPanel; ++k) li[k] = pan[col(kb, k) + i];
 #pragma unroll
         for (int c = 0; c < KC; ++c) {
-          if (j0 + c < c1 && i >= j0 + c) {
+          if (j0 + c < P && i >= j0 + c) {
             T a0 = T(0), a1 = T(0);  // two half-length FMA chains per output
 #pragma unroll
             for (int k = 0; k < kPanel; k += 2) {
@@ -208,18 +285,18 @@ __device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *
       }
     }
   };
-  // right-looking with one block of look-ahead: once block kb's rows are solved, the
-  // next block's columns take its update first; then warp 0 factors the next diagonal
-  // block while the other warps update the remaining columns.  Every element takes
-  // the same updates in the same order as without the look-ahead.
+  // right-looking with one block of look-ahead: once block kb's rows are solved, the next
+  // diagonal block takes its update first; then warp 0 factors it while the other warps update
+  // the rest (and, FP32, warp 1 inverts block kb).
   if (warp == 0) factor_diag(0);
   __syncthreads();
   if (*fail_s) return;
-  for (int kb = 0; kb < P; kb += kPanel) {
-    const int ke = min(kb + kPanel, P), w = ke - kb;
+  int kb = 0;
+  for (; kb + kPanel < P; kb += kPanel) {  // (rows below exist only under a full block)
+    const int ke = kb + kPanel, ke2 = min(ke + kPanel, P);
     // rows below the block: L(i, kb:ke) = S(i, kb:ke) L_D^-T
-    if constexpr (std::is_same<T, double>::value) {
-      if (ke >= P) break;  // (rows below exist only under a full block)
+    const T *pan = Lm + cb[kb];  // the panel: column c of it at pan + col(kb, c)
+    if constexpr (kF64) {
       // four lanes per row, lane q holding columns q, q + 4, ..: 36 + 4 FP64 instructions a warp
       // however few rows are left (136 with a thread per row)
       const int q = lane & 3;
@@ -239,76 +316,72 @@ __device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *
         for (int c = 0; c < 4; ++c)
           if (i < P) Lm[ix(i, kb + q + 4 * c)] = u[c] * dinv[kb + q + 4 * c];
       }
-      // trailing update, an element of the packed triangle per lane, so that no lane idles at the
-      // columns' ends (a warp per two columns kept 40 to 75 % of them busy); behind the next
-      // block's columns the warps draw 32 elements at a time, warp 0 once it has factored
-      const int R = P - ke, n = R * (R + 1) / 2, w2 = min(kPanel, R), n1 = w2 * R - w2 * (w2 - 1) / 2;
-      T *tri = Lm + ix(ke, ke);
-      int cbk[kPanel];
+    } else {
+      const float *src = Ld[(kb / kPanel) & 1], *r = ri[(kb / kPanel) & 1];
+      for (int i = ke + tid; i < P; i += nt) {
+        float v[kPanel];
 #pragma unroll
-      for (int c = 0; c < kPanel; ++c) cbk[c] = cb[kb + c];
-      auto update = [&](int o) {
-        const int r = n - 1 - o;  // from the end: column P - 1 - jj holds jj + 1 elements
-        int jj = (int)((sqrtf(8.f * (float)r + 1.f) - 1.f) * 0.5f);
-        jj += (jj + 1) * (jj + 2) / 2 <= r;
-        jj -= jj * (jj + 1) / 2 > r;
-        const int j = P - 1 - jj, i = P - 1 - (r - jj * (jj + 1) / 2);
-        double a0 = 0.0, a1 = 0.0;
+        for (int c = 0; c < kPanel; ++c) v[c] = pan[col(kb, c) + i];
 #pragma unroll
-        for (int k = 0; k < kPanel; k += 2) {
-          a0 += Lm[cbk[k] + i] * Lm[cbk[k] + j];
-          a1 += Lm[cbk[k + 1] + i] * Lm[cbk[k + 1] + j];
+        for (int c = 0; c < kPanel; ++c) {
+          v[c] *= r[c];
+#pragma unroll
+          for (int q = (c + 1) / 4; q < kPanel / 4; ++q) {
+            const float4 l = *reinterpret_cast<const float4 *>(src + c * kPanel + 4 * q);
+            const float lv[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+              if (4 * q + m > c) v[4 * q + m] = fmaf(-v[c], lv[m], v[4 * q + m]);
+          }
         }
-        tri[o] -= a0 + a1;
-      };
-      __syncthreads();
-      for (int o = tid; o < n1; o += nt) update(o);
-      if (tid == 0) drawn = n1;
-      __syncthreads();
-      if (warp == 0) factor_diag(ke);
-      for (;;) {
+#pragma unroll
+        for (int c = 0; c < kPanel; ++c) Lm[cb[kb] + col(kb, c) + i] = v[c];
+      }
+    }
+    __syncthreads();
+    auto update = [&](int i, int j) {
+      T a0 = T(0), a1 = T(0);
+#pragma unroll
+      for (int k = 0; k < kPanel; k += 2) {
+        a0 += pan[col(kb, k) + i] * pan[col(kb, k) + j];
+        a1 += pan[col(kb, k + 1) + i] * pan[col(kb, k + 1) + j];
+      }
+      Lm[ix(i, j)] -= a0 + a1;
+    };
+    for (int o = tid; o < kPanel * kPanel; o += nt) {  // the next diagonal block
+      const int i = ke + o / kPanel, j = ke + o % kPanel;
+      if (i < P && j <= i) update(i, j);
+    }
+    if (kF64 && tid == 0) drawn = 0;
+    __syncthreads();
+    if (warp == 0) factor_diag(ke);
+    if constexpr (kF64) {
+      // an element of the packed triangle per lane, so that no lane idles at the columns' ends (a
+      // warp per two columns kept 40 to 75 % of them busy); the warps draw 32 elements at a time,
+      // warp 0 once it has factored
+      const int R = P - ke, n = R * (R + 1) / 2;
+      // (on few elements a warp on warp 0's quarter of the SM would only delay it)
+      while (warp == 0 || warp % 4 != 0 || n > kDrawAll) {
         int o = 0;
         if (lane == 0) o = atomicAdd(&drawn, 32);
         o = __shfl_sync(0xffffffffu, o, 0);
         if (o >= n) break;
-        if (o + lane < n) update(o + lane);
+        o += lane;
+        if (o < n) element(P, n, o, ke2, update);
       }
     } else {
-      int cbk[kPanel];
-#pragma unroll
-      for (int c = 0; c < kPanel; ++c) cbk[c] = c < w ? cb[kb + c] : 0;
-      for (int i = ke + tid; i < P; i += nt) {
-        T r[kPanel];
-#pragma unroll
-        for (int c = 0; c < kPanel; ++c) r[c] = c < w ? Lm[cbk[c] + i] : T(0);
-#pragma unroll
-        for (int c = 0; c < kPanel; ++c) {
-          if (c < w) {
-            T v = r[c];
-#pragma unroll
-            for (int m = 0; m < c; ++m) v -= r[m] * Lm[ix(kb + c, kb + m)];
-            r[c] = v * dinv[kb + c];
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < kPanel; ++c)
-          if (c < w) Lm[cbk[c] + i] = r[c];
-      }
-      __syncthreads();
-      if (ke >= P) break;
-      const int ke2 = min(ke + kPanel, P);
-      update_cols(std::integral_constant<int, 2>{}, cbk, w, ke, ke2, warp, nw);  // the next block's columns
-      __syncthreads();
-      if (warp == 0)
-        factor_diag(ke);
-      else
-        update_cols(std::integral_constant<int, 4>{}, cbk, w, ke2, P, warp - 1, nw - 1);
+      if (warp == 1) invert_diag(kb);
+      if (warp >= 1) update_cols(kb, ke, ke2, warp - 1, nw - 1);
     }
     __syncthreads();
     if (*fail_s) return;
   }
+  if (!kF64) {
+    if (warp == 0) invert_diag(kb);
+    __syncthreads();
+  }
   for (int it = 0; it <= refine; ++it) {
-    chol_substitute<T>(Lm, cb, y, dinv, tmp, P);
+    chol_substitute<T>(Lm, cb, y, dinv, P);
     for (int i = tid; i < P; i += nt) x[i] += (double)y[i];
     __syncthreads();
     if (it == refine) break;
@@ -420,12 +493,11 @@ __device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *
 
 #undef ix
 
-// store: keep the packed factor and the pivots in wv.facs for the refinement solves
+// store: keep the packed factor in wv.facs for the refinement solves
 template <typename T>
-__global__ void __launch_bounds__(256) k_factor_solve(PlanView pv, WorkView wv, int refine, int store) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_factor_solve(PlanView pv, WorkView wv, int refine, int store) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int fail_s;
-  __shared__ T tmp_s[kPanel];
   const int b = pv.fs_prob[blockIdx.x];
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   const int N = pv.p_npose[b], P = 6 * N;
@@ -451,17 +523,16 @@ __global__ void __launch_bounds__(256) k_factor_solve(PlanView pv, WorkView wv, 
   T *colacc = reinterpret_cast<T *>(reinterpret_cast<unsigned char *>(dinv) + (((size_t)P * sizeof(T) + 15) & ~(size_t)15));
   for (int j = threadIdx.x; j < P; j += blockDim.x) cb[j] = j * P - (j * (j + 1)) / 2;
   __syncthreads();
-  factor_solve_body<T>(Lm, cb, y, x, xs, dinv, tmp_s, colacc, A, SL, g, gL, lam, P, refine, &fail_s);
+  factor_solve_body<T>(Lm, cb, y, x, xs, dinv, colacc, A, SL, g, gL, lam, P, refine, &fail_s);
   __syncthreads();
   const bool failed = fail_s != 0;
   for (int i = threadIdx.x; i < P; i += blockDim.x) wv.delta[po + i] = failed ? 0.0 : x[i];
   if (threadIdx.x == 0) wv.lm[b].ref_done = 0;  // this step's refinement starts afresh
   if (threadIdx.x == 0 && failed) atomicOr(&wv.lm[b].fail, FAIL_PIVOT);
   if constexpr (std::is_same<T, float>::value) {
-    if (store && !failed) {  // packed factor, then the pivots' reciprocals
+    if (store && !failed) {
       float *dst = wv.facs + off;
       for (size_t k = threadIdx.x; k < npk; k += blockDim.x) dst[k] = Lm[k];
-      for (int k = threadIdx.x; k < P; k += blockDim.x) dst[npk + k] = dinv[k];
     }
   }
   // clear the consumed S_L tiles (every element whose row tile >= column tile) and g_L
