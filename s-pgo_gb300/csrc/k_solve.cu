@@ -57,7 +57,7 @@ __device__ __forceinline__ void element(int P, int n, int o, int r0, F &&f) {
 // Bound by the diagonal blocks' chain and the barriers in FP32 (one 10-pose window: 35 us with a
 // pivot, its root, its reciprocal and fifteen shuffles per column, the factor's columns found
 // through a table and two barriers per block of the substitutions; 18.4 us so; 64 windows of up to
-// 32 poses: 115 and 83 us) and in FP64 by the FP64 pipe's 2 FMA per cycle and SM (eight solves of
+// 32 poses: 115 and 69 us) and in FP64 by the FP64 pipe's 2 FMA per cycle and SM (eight solves of
 // a 10-pose window: 613 us with a thread per row, a warp per two columns and a row's columns in
 // one lane; 300 us laid out by FP64 instructions as below).
 // `refine` iterative-refinement steps form the residual g_S - S x (double-float on the FP32 path,
@@ -253,35 +253,62 @@ __device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *
         if (lane <= k && k < w) Lm[ix(kb + k, kb + lane)] = v[k];
     }
   };
-  // FP32: the update of columns [c0, P), rows from max(j, r0), with the finished block kb: warp wi
-  // of nwu, four columns per warp pass (each loaded panel row serves four columns; an element per
-  // thread, which reads eight times as much of the panel, cost 64 windows of up to 32 poses 5 % and
-  // gained a 10-pose window nothing)
-  auto update_cols = [&](int kb, int c0, int r0, int wi, int nwu) {
-    const T *pan = Lm + cb[kb];
-    constexpr int KC = 4;
-    for (int j0 = c0 + KC * wi; j0 < P; j0 += KC * nwu) {
-      T ljk[KC][kPanel];
+  // FP32: the update of all below and beside the next diagonal block with the solved panel, which
+  // the row solves also left in `stage` (column k's rows from ke at stage + k ld): warp wi of nwu,
+  // tiles of 32 rows and 16 columns, four by four per lane (rows lr + 8 a, columns 4 lc + b), so
+  // that 16 FMAs take five shared-memory accesses.  (Four columns per warp pass with a lane per
+  // row, 24 accesses for 64 FMAs and the columns' own 64, took 24k cycles for the first block of a
+  // 32-pose window, 12.4k so; an element per lane, 32 for 16, 5 % longer still.)
+  float *stage = reinterpret_cast<float *>(colacc);  // free until the residual
+  const int ld = (P + 3) & ~3;
+  auto update_tiles = [&](int ke, int wi, int nwu) {
+    if constexpr (!kF64) {
+    const int R = P - ke, lr = lane & 7, lc = lane >> 3;
+    int turn = wi;
+    for (int j0 = 0; j0 < R; j0 += 16)
+      for (int i0 = j0 & ~31; i0 < R; i0 += 32) {
+        if (turn-- != 0) continue;
+        turn = nwu - 1;
+        // (rows and columns past the end take the last one's place and are dropped)
+        const float *cols = stage + min(j0 + 4 * lc, ld - 4);
+        const float *rows[4];
 #pragma unroll
-      for (int c = 0; c < KC; ++c)
+        for (int a = 0; a < 4; ++a) rows[a] = stage + min(i0 + lr + 8 * a, R - 1);
+        float acc[4][4] = {};
 #pragma unroll
-        for (int k = 0; k < kPanel; ++k) ljk[c][k] = pan[col(kb, k) + min(j0 + c, P - 1)];
-      for (int i = max(j0, r0) + lane; i < P; i += 32) {
-        T li[kPanel];
+        for (int k0 = 0; k0 < kPanel; k0 += 4) {  // (loads of four columns first)
+          float4 c[4];
+          float x[4][4];
 #pragma unroll
-        for (int k = 0; k < kPanel; ++k) li[k] = pan[col(kb, k) + i];
+          for (int q = 0; q < 4; ++q) {
+            c[q] = *reinterpret_cast<const float4 *>(cols + (k0 + q) * ld);
 #pragma unroll
-        for (int c = 0; c < KC; ++c) {
-          if (j0 + c < P && i >= j0 + c) {
-            T a0 = T(0), a1 = T(0);  // two half-length FMA chains per output
-#pragma unroll
-            for (int k = 0; k < kPanel; k += 2) {
-              a0 += li[k] * ljk[c][k];
-              a1 += li[k + 1] * ljk[c][k + 1];
-            }
-            Lm[cb[j0 + c] + i] -= a0 + a1;
+            for (int a = 0; a < 4; ++a) x[q][a] = rows[a][(k0 + q) * ld];
           }
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+              acc[a][0] = fmaf(x[q][a], c[q].x, acc[a][0]);
+              acc[a][1] = fmaf(x[q][a], c[q].y, acc[a][1]);
+              acc[a][2] = fmaf(x[q][a], c[q].z, acc[a][2]);
+              acc[a][3] = fmaf(x[q][a], c[q].w, acc[a][3]);
+            }
         }
+        float *dst[4], old[4][4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          dst[b] = Lm + ix(ke + i0 + lr, ke + min(j0 + 4 * lc + b, R - 1));
+#pragma unroll
+          for (int a = 0; a < 4; ++a) old[a][b] = dst[b][min(8 * a, R - 1 - i0 - lr)];
+        }
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            const int i = i0 + lr + 8 * a;
+            if (i >= j0 + 4 * lc + b && i >= kPanel && i < R) dst[b][8 * a] = old[a][b] - acc[a][b];
+          }
       }
     }
   };
@@ -335,7 +362,10 @@ __device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *
           }
         }
 #pragma unroll
-        for (int c = 0; c < kPanel; ++c) Lm[cb[kb] + col(kb, c) + i] = v[c];
+        for (int c = 0; c < kPanel; ++c) {
+          Lm[cb[kb] + col(kb, c) + i] = v[c];
+          stage[c * ld + i - ke] = v[c];
+        }
       }
     }
     __syncthreads();
@@ -371,7 +401,7 @@ __device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *
       }
     } else {
       if (warp == 1) invert_diag(kb);
-      if (warp >= 1) update_cols(kb, ke, ke2, warp - 1, nw - 1);
+      if (warp >= 1) update_tiles(ke, warp - 1, nw - 1);
     }
     __syncthreads();
     if (*fail_s) return;
@@ -495,7 +525,7 @@ __device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *
 
 // store: keep the packed factor in wv.facs for the refinement solves
 template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_factor_solve(PlanView pv, WorkView wv, int refine, int store) {
+__global__ void __launch_bounds__(256) k_factor_solve(PlanView pv, WorkView wv, int refine, int store) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int fail_s;
   const int b = pv.fs_prob[blockIdx.x];
