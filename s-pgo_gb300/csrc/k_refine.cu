@@ -66,38 +66,38 @@ __device__ __forceinline__ bool refine_active(const WorkView &wv, int b) {
 // convention of the pose blocks, k_system.cu).  With the prefix sums
 // Om(k) = sum_{i<k} R_i psi_i and V(k) = sum_{i<k} c_i x R_i psi_i + R_i rho_i,
 // W(lo, hi) = [Om(hi) - Om(lo) ; V(hi) - V(lo) - c_lo x (Om(hi) - Om(lo))].
-// Only differences of the prefix sums enter, so a CTA takes kTwSlice consecutive lo's and
-// sums over their own poses and the D after them: a batch's windows are one CTA each, a long
-// trajectory spreads over the GPU (500 poses: 141 us on one SM's FP64 pipe, 12 us spread out).
-constexpr int kTwThreads = 128;
+// Only differences of the prefix sums enter, so a CTA takes a slice of consecutive lo's and
+// sums over their own poses and the D after them; the slices are as long as still gives every SM a
+// CTA (kTwSlice at most), so that a batch's windows are one CTA each and few windows or a long
+// trajectory spread over the GPU (500 poses: 141 us on one SM's FP64 pipe, 12 us spread out).
+// Bound by FP64 instructions, 64 cycles each for a quarter of an SM, so every phase spreads over
+// all four (64 windows of up to 32 poses, two slices each: 11.5 us with a thread per pose and a
+// slice per window, 7.5 us so).
+constexpr int kTwThreads = 192;  // (six warps: one per component in the scan)
 constexpr int kTwSlice = 32;
 
-__global__ void __launch_bounds__(kTwThreads) k_pair_twists(PlanView pv, WorkView wv) {
+__global__ void __launch_bounds__(kTwThreads) k_pair_twists(PlanView pv, WorkView wv, int slice) {
   __shared__ double tw_s[(kTwSlice + SPGO_MAX_WINDOW + 1) * 6];
-  const int b = blockIdx.x, l0 = kTwSlice * blockIdx.y;
+  const int b = blockIdx.x, l0 = slice * blockIdx.y;
   const int N = pv.p_npose[b], D = pv.p_pair_D[b], fo = pv.p_frame_off[b], po = pv.p_param_off[b];
   if (l0 >= N || !refine_active(wv, b)) return;
-  const int n = min(N - l0, kTwSlice + D);  // the slice's poses and the D after them
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const float *Rh = wv.fr_Rf + (size_t)(fo + l0 + i) * 18, *Rl = wv.fr_Rl + (size_t)(fo + l0 + i) * 18;
-    const double *c = wv.fr_c + (size_t)(fo + l0 + i) * 6;
+  const int n = min(N - l0, slice + D);  // the slice's poses and the D after them
+  for (int t = threadIdx.x; t < 3 * n; t += blockDim.x) {  // thread per (pose, row)
+    const int i = t / 3, r = t % 3;
+    const float *Rh = wv.fr_Rf + (size_t)(fo + l0 + i) * 18 + 3 * r, *Rl = wv.fr_Rl + (size_t)(fo + l0 + i) * 18 + 3 * r;
     const double *x = wv.delta + po + 6 * (l0 + i);
-    double w[3], v[3];
+    double R[3];
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      double R[3];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) R[k] = (double)Rh[3 * r + k] + (double)Rl[3 * r + k];
-      w[r] = R[0] * x[0] + R[1] * x[1] + R[2] * x[2];
-      v[r] = R[0] * x[3] + R[1] * x[4] + R[2] * x[5];
-    }
+    for (int k = 0; k < 3; ++k) R[k] = (double)Rh[k] + (double)Rl[k];
+    tw_s[(size_t)(i + 1) * 6 + r] = R[0] * x[0] + R[1] * x[1] + R[2] * x[2];
+    tw_s[(size_t)(i + 1) * 6 + 3 + r] = R[0] * x[3] + R[1] * x[4] + R[2] * x[5];
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < 3 * n; t += blockDim.x) {
+    const int i = t / 3, k = t % 3, k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1;
+    const double *c = wv.fr_c + (size_t)(fo + l0 + i) * 6;
     double *o = tw_s + (size_t)(i + 1) * 6;
-    o[0] = w[0];
-    o[1] = w[1];
-    o[2] = w[2];
-    o[3] = v[0] + (c[1] * w[2] - c[2] * w[1]);
-    o[4] = v[1] + (c[2] * w[0] - c[0] * w[2]);
-    o[5] = v[2] + (c[0] * w[1] - c[1] * w[0]);
+    o[3 + k] += c[k1] * o[k2] - c[k2] * o[k1];
   }
   if (threadIdx.x < 6) tw_s[threadIdx.x] = 0.0;
   __syncthreads();
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kTwThreads) k_pair_twists(PlanView pv, WorkVie
   }
   __syncthreads();
   float *out = wv.twist + ((size_t)pv.p_pair_off[b] + (size_t)l0 * D) * 6;
-  for (int t = threadIdx.x; t < min(kTwSlice, N - l0) * D; t += blockDim.x) {
+  for (int t = threadIdx.x; t < min(slice, N - l0) * D; t += blockDim.x) {
     const int lo = t / D, hi = lo + t % D + 1;  // relative to l0
     if (l0 + hi > N) continue;
     const double *c = wv.fr_c + (size_t)(fo + l0 + lo) * 6;
@@ -139,8 +139,10 @@ __global__ void __launch_bounds__(kTwThreads) k_pair_twists(PlanView pv, WorkVie
 }
 
 int launch_pair_twists(const PlanView &pv, const WorkView &wv, void *stream) {
-  const int slices = (pv.max_P / 6 + kTwSlice - 1) / kTwSlice;
-  k_pair_twists<<<dim3(pv.B, slices), kTwThreads, 0, (cudaStream_t)stream>>>(pv, wv);
+  const int nmax = pv.max_P / 6;
+  int slice = kTwSlice;
+  while (slice > 8 && (long long)pv.B * ((nmax + slice - 1) / slice) < 152) slice /= 2;
+  k_pair_twists<<<dim3(pv.B, (nmax + slice - 1) / slice), kTwThreads, 0, (cudaStream_t)stream>>>(pv, wv, slice);
   ++g_launches;
   return (int)cudaGetLastError();
 }
@@ -473,7 +475,9 @@ int launch_resid_pass(const PlanView &pv, const WorkView &wv, const Params &prm,
 // that sum is the prefix sum of diff up to i.  Then r(i) = [R_i^T (.)_w ; R_i^T (.)_v].
 // The row sums (fixed lo) re-centre linearly: sum_hi n = sum_hi m_w + c_lo x sum_hi m_v;
 // the column sums (fixed hi) take c_lo x m_v per record.  One thread per (row or column,
-// component), no atomics.
+// component), no atomics.  Bound by FP64 instructions (64 cycles of a quarter SM each) and the
+// substitutions' chain: 64 windows of up to 32 poses 29.2 us with a serial prefix, a thread per
+// pose in the right-hand side and warps that ran through rows and columns alike, 19.7 us so.
 constexpr int kRsThreads = 256;
 
 // shared memory: centres, row and column sums | cb | y | the packed factor
@@ -531,75 +535,91 @@ __global__ void __launch_bounds__(kRsThreads) k_resid_solve(PlanView pv, WorkVie
     cs[k] = wv.fr_c[(size_t)(fo + k / 3) * 6 + k % 3];
   __syncthreads();
   double *recs = wv.pdual + (size_t)pv.p_pair_off[b] * 6;
-  for (int t = tid; t < 12 * N; t += nt) {
-    const int k = t % 6;
-    if (t < 6 * N) {  // row lo = t / 6
-      const int lo = t / 6;
+  // Three kinds of sums, each from a warp's first lane on, so that no warp runs through two kinds:
+  // rows (all components), columns' m_v, and columns' m_w with the records moved from c_lo.
+  const int w_row = (6 * N + 31) / 32, w_col = (3 * N + 31) / 32, lane = tid & 31;
+  for (int w = tid >> 5; w < w_row + 2 * w_col; w += nt >> 5) {
+    if (w < w_row) {
+      const int t = 32 * w + lane, lo = t / 6, k = t % 6;
+      if (lo >= N) continue;
       const double *r = recs + (size_t)lo * D * 6 + k;
       const int nd = min(D, N - lo);
       double acc = 0.0;
-#pragma unroll 4
+#pragma unroll 8
       for (int d = 0; d < nd; ++d) acc += r[(size_t)d * 6];
       rowm[lo * 6 + k] = acc;
-    } else {  // column hi = (t - 6 N) / 6 + 1
-      const int hi = (t - 6 * N) / 6 + 1;
-      double acc = 0.0;
-      if (k < 3) {
-        const int k1 = (k + 1) % 3, k2 = (k + 2) % 3;
+      continue;
+    }
+    const bool moved = w >= w_row + w_col;
+    const int t = 32 * (w - w_row - (moved ? w_col : 0)) + lane, hi = t / 3 + 1, k = t % 3;
+    if (hi > N) continue;
+    double acc = 0.0;
+    if (moved) {
+      const int k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1;
 #pragma unroll 4
-        for (int lo = max(0, hi - D); lo < hi; ++lo) {
-          const double *r = recs + ((size_t)lo * D + (hi - lo - 1)) * 6;
-          acc += r[k] + (cs[lo * 3 + k1] * r[3 + k2] - cs[lo * 3 + k2] * r[3 + k1]);
-        }
-      } else {
-#pragma unroll 4
-        for (int lo = max(0, hi - D); lo < hi; ++lo) acc += recs[((size_t)lo * D + (hi - lo - 1)) * 6 + k];
+      for (int lo = max(0, hi - D); lo < hi; ++lo) {
+        const double *r = recs + ((size_t)lo * D + (hi - lo - 1)) * 6;
+        acc = fma(-cs[lo * 3 + k2], r[3 + k1], fma(cs[lo * 3 + k1], r[3 + k2], acc + r[k]));
       }
       colm[hi * 6 + k] = acc;
+    } else {
+#pragma unroll 8
+      for (int lo = max(0, hi - D); lo < hi; ++lo) acc += recs[((size_t)lo * D + (hi - lo - 1)) * 6 + 3 + k];
+      colm[hi * 6 + 3 + k] = acc;
     }
   }
   if (tid < 6) colm[tid] = 0.0;  // no record ends at pose 0
   __syncthreads();
   for (size_t k = tid; k < (size_t)N * D * 6; k += nt) recs[k] = 0.0;  // cleared for the next pass
-  if (tid < 6) {  // prefix sums over the poses; rowm(i) becomes the sum of the records covering pose i
-    const int k = tid, k1 = (k + 1) % 3, k2 = (k + 2) % 3;
-    double acc = 0.0;
-    for (int i = 0; i < N; ++i) {
-      const double *c = cs + i * 3;
-      const double *m = rowm + i * 6;
-      const double nrow = k < 3 ? m[k] + (c[k1] * m[3 + k2] - c[k2] * m[3 + k1]) : m[k];
-      acc += nrow - colm[i * 6 + k];
-      __syncwarp(0x3fu);
-      rowm[i * 6 + k] = acc;  // every lane has read row i's m_v above
+  // pose i's term: its row sums moved from c_i, less the column sums of the records ending there
+  for (int t = tid; t < 6 * N; t += nt) {
+    const int i = t / 6, k = t % 6, k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1;
+    const double *m = rowm + i * 6, *c = cs + i * 3;
+    double v = m[k] - colm[t];
+    if (k < 3) v = fma(-c[k2], m[3 + k1], fma(c[k1], m[3 + k2], v));
+    colm[t] = v;  // (read and written by this thread alone)
+  }
+  __syncthreads();
+  // its prefix over the poses, a warp per component: the sum of the records covering pose i
+  for (int k = tid >> 5; k < 6; k += nt >> 5) {
+    double carry = 0.0;
+    for (int s = 0; s < N; s += 32) {
+      double v = s + lane < N ? colm[(s + lane) * 6 + k] : 0.0;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const double u = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += u;
+      }
+      v += carry;
+      if (s + lane < N) rowm[(s + lane) * 6 + k] = v;
+      carry = __shfl_sync(0xffffffffu, v, 31);
     }
+  }
+  __syncthreads();
+  for (int t = tid; t < 3 * N; t += nt) {  // m_w about c_i
+    const int i = t / 3, k = t % 3, k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1;
+    const double *c = cs + i * 3;
+    double *S = rowm + i * 6;
+    S[k] -= c[k1] * S[3 + k2] - c[k2] * S[3 + k1];
   }
   __syncthreads();
   float *y = reinterpret_cast<float *>(smem_raw + o_y);
   const double lam = wv.lm[b].lam;
   const float *A = reinterpret_cast<const float *>(wv.A) + pv.p_S_off[b];
-  for (int i = tid; i < N; i += nt) {
-    double R[9], ci[3];
-    frame_Rc(wv, fo + i, R, ci);
-    const double *S = rowm + i * 6;
-    const double w[3] = {S[0] - (ci[1] * S[5] - ci[2] * S[4]), S[1] - (ci[2] * S[3] - ci[0] * S[5]),
-                         S[2] - (ci[0] * S[4] - ci[1] * S[3])};
-    double out[6];
+  for (int p = tid; p < P; p += nt) {  // R_i^T of both halves, a thread per unknown
+    const int i = p / 6, k = p % 6, r = k < 3 ? k : k - 3;
+    const float *Rh = wv.fr_Rf + (size_t)(fo + i) * 18 + r, *Rl = wv.fr_Rl + (size_t)(fo + i) * 18 + r;
+    const double *S = rowm + i * 6 + (k < 3 ? 0 : 3);
+    double out = 0.0;
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      out[r] = R[r] * w[0] + R[3 + r] * w[1] + R[6 + r] * w[2];
-      out[3 + r] = R[r] * S[3] + R[3 + r] * S[4] + R[6 + r] * S[5];
-    }
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      const int p = 6 * i + k;
-      const double x = wv.delta[po + p];
-      const double rhs = out[k] - lam * (double)A[(size_t)p * P + p] * x - (double)wv.rhsB[po + p];
-      wv.rhsB[po + p] = 0.f;
-      if (small)
-        y[p] = (float)rhs;
-      else
-        reinterpret_cast<float *>(wv.lg_y)[po + p] = (float)rhs;
-    }
+    for (int q = 0; q < 3; ++q) out += ((double)Rh[3 * q] + (double)Rl[3 * q]) * S[q];
+    const double x = wv.delta[po + p];
+    const double rhs = out - lam * (double)A[(size_t)p * P + p] * x - (double)wv.rhsB[po + p];
+    wv.rhsB[po + p] = 0.f;
+    if (small)
+      y[p] = (float)rhs;
+    else
+      reinterpret_cast<float *>(wv.lg_y)[po + p] = (float)rhs;
   }
   if (!small) return;  // the multi-CTA substitutions (k_chol_large.cu) follow
   int *cb = reinterpret_cast<int *>(smem_raw + o_cb);
