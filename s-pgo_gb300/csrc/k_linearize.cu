@@ -321,139 +321,101 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_cost(PlanView p
 // precision of the FP32 path's frame tables: fr_Rf + fr_Rl, fr_ch + fr_cl), on the
 // FP32 pipes instead of FP64 (which runs at a small fraction of their rate on
 // this GPU).  Writes only the tables the FP32 kernels read.
-__device__ __forceinline__ void compose34_df(const df *A, const df *B, df *C) {
+// row p of a product P M
+__device__ __forceinline__ void compose_row_df(const df *p, const df *M, df *o) {
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      df v = df_dot3(A[4 * i].h, A[4 * i].l, A[4 * i + 1].h, A[4 * i + 1].l, A[4 * i + 2].h, A[4 * i + 2].l,
-                     B[j], B[4 + j], B[8 + j]);
-      if (j == 3) v = v + A[4 * i + 3];
-      C[4 * i + j] = v;
-    }
-  }
+  for (int j = 0; j < 4; ++j) o[j] = df_dot3(p[0].h, p[0].l, p[1].h, p[1].l, p[2].h, p[2].l, M[j], M[4 + j], M[8 + j]);
+  o[3] = o[3] + p[3];
 }
 
-// (also the left centre as FP64, h + l, which the refinement's FP64 sums read)
-__device__ __forceinline__ void write_frame_df(const WorkView &wv, size_t f, const df *G, const df *Trl) {
-  df Gr[12];
-  compose34_df(G, Trl, Gr);
+// row r of frame f, G its 3x4 pose (also the left centre as FP64, h + l, which the refinement's
+// FP64 sums read)
+__device__ __forceinline__ void write_frame_row_df(const WorkView &wv, size_t f, int r, const df *G, const df *Trl) {
+  df Gr[4];
+  compose_row_df(G, Trl, Gr);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      wv.fr_Rf[f * 18 + 3 * i + j] = G[4 * i + j].h;
-      wv.fr_Rf[f * 18 + 9 + 3 * i + j] = Gr[4 * i + j].h;
-      wv.fr_Rl[f * 18 + 3 * i + j] = G[4 * i + j].l;
-      wv.fr_Rl[f * 18 + 9 + 3 * i + j] = Gr[4 * i + j].l;
-    }
-    wv.fr_ch[f * 6 + i] = G[4 * i + 3].h;
-    wv.fr_ch[f * 6 + 3 + i] = Gr[4 * i + 3].h;
-    wv.fr_cl[f * 6 + i] = G[4 * i + 3].l;
-    wv.fr_cl[f * 6 + 3 + i] = Gr[4 * i + 3].l;
-    wv.fr_c[f * 6 + i] = (double)G[4 * i + 3].h + (double)G[4 * i + 3].l;
+  for (int j = 0; j < 3; ++j) {
+    const size_t q = f * 18 + 3 * r + j;
+    wv.fr_Rf[q] = G[j].h;
+    wv.fr_Rf[q + 9] = Gr[j].h;
+    wv.fr_Rl[q] = G[j].l;
+    wv.fr_Rl[q + 9] = Gr[j].l;
   }
+  const size_t q = f * 6 + r;
+  wv.fr_ch[q] = G[3].h;
+  wv.fr_ch[q + 3] = Gr[3].h;
+  wv.fr_cl[q] = G[3].l;
+  wv.fr_cl[q + 3] = Gr[3].l;
+  wv.fr_c[q] = (double)G[3].h + (double)G[3].l;
 }
 
-// M_k <- M_0 M_1 ... M_k over the first n lanes of a warp (earlier factors on the left)
-__device__ __forceinline__ void scan34_df(df *M, int lane, int n) {
-#pragma unroll 1
-  for (int d = 1; d < n; d <<= 1) {
-    df P[12];
-#pragma unroll
-    for (int q = 0; q < 12; ++q)
-      P[q] = df{__shfl_up_sync(0xffffffffu, M[q].h, d), __shfl_up_sync(0xffffffffu, M[q].l, d)};
-    if (lane >= d) {
-      df C[12];
-      compose34_df(P, M, C);
-#pragma unroll
-      for (int q = 0; q < 12; ++q) M[q] = C[q];
-    }
-  }
-}
+// As k_chain, one CTA per problem, three threads (rows) per frame, up to kChainDfFrames frames a
+// pass (in place: two barriers per step of the scan).  Bound by the scan's latency: 10 poses 8.3 us
+// and 500 poses 36 us with a lane per frame, 5.3 and 24 us so (a row is a third of a frame).
+constexpr int kChainDfFrames = 256;
 
-// One CTA per problem, 32 frames a warp (one warp for the windows of a batch, up to
-// kChainWarps for a long trajectory): each warp scans its frames, warp 0 scans the warps'
-// totals onto the carry of the pass before.  The chain is latency: one warp walking 500
-// poses in 16 passes took 135 us, eight warps in two passes 36 us (one 20-pose window: 13.8 -> 9.0 us).
-constexpr int kChainWarps = 8;
-
-__global__ void __launch_bounds__(32 * kChainWarps) k_chain_df(PlanView pv, WorkView wv,
-                                                               const double *__restrict__ poses, int gate) {
-  __shared__ df tot[kChainWarps][12];   // a warp's product, then everything before it
-  __shared__ df carry_s[12];
+__global__ void __launch_bounds__(3 * kChainDfFrames) k_chain_df(PlanView pv, WorkView wv,
+                                                                 const double *__restrict__ poses, int gate) {
   const int b = blockIdx.x;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   if (!problem_active(wv.lm, b, gate)) return;
+  __shared__ df buf[kChainDfFrames][12];
+  __shared__ df Trl[12], last[12];
   const int N = pv.p_npose[b], fo = pv.p_frame_off[b], po = pv.p_pose_off[b];
-  df Trl[12], carry[12];
-  {
-    const df t = df_from_double(pv.p_Trl[12 * b + min(lane, 11)]);  // lane q converts entry q for the warp
+  const int nf = blockDim.x / 3, f = threadIdx.x / 3, r = threadIdx.x % 3;
+  if (threadIdx.x < 12) Trl[threadIdx.x] = df_from_double(pv.p_Trl[12 * b + threadIdx.x]);
+  for (int s = 0; s < N; s += nf) {
+    const int k = s + f, n = min(nf, N - s);
+    if (k < N) {  // row r of the pose, for its inverse [R^T, -R^T t]
+      const double *T = poses + 12 * (size_t)(po + k) + 4 * r;
 #pragma unroll
-    for (int q = 0; q < 12; ++q) {
-      Trl[q] = df{__shfl_sync(0xffffffffu, t.h, q), __shfl_sync(0xffffffffu, t.l, q)};
-      carry[q] = df_make((q == 0 || q == 5 || q == 10) ? 1.f : 0.f);
+      for (int j = 0; j < 4; ++j) buf[f][4 * r + j] = df_from_double(T[j]);
     }
-  }
-  if (threadIdx.x == 0) write_frame_df(wv, (size_t)fo, carry, Trl);
-  for (int s = 0; s < N; s += 32 * nw) {
-    const int k = s + threadIdx.x;
-    df M[12];
-#pragma unroll
-    for (int q = 0; q < 12; ++q) M[q] = df_make((q == 0 || q == 5 || q == 10) ? 1.f : 0.f);
-    if (k < N) {  // inverse of the incremental pose: [R^T, -R^T t]
-      const double *T = poses + 12 * (size_t)(po + k);
-      df Td[12];
-#pragma unroll
-      for (int q = 0; q < 12; ++q) Td[q] = df_from_double(T[q]);
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-#pragma unroll
-        for (int j = 0; j < 3; ++j) M[4 * i + j] = Td[4 * j + i];
-        M[4 * i + 3] = -df_dot3(Td[i].h, Td[i].l, Td[4 + i].h, Td[4 + i].l, Td[8 + i].h, Td[8 + i].l, Td[3], Td[7],
-                                Td[11]);
-      }
+    __syncthreads();
+    if (s == 0 && f == 0) {
+      const df I[4] = {df_make(r == 0 ? 1.f : 0.f), df_make(r == 1 ? 1.f : 0.f), df_make(r == 2 ? 1.f : 0.f), df_make(0.f)};
+      write_frame_row_df(wv, (size_t)fo, r, I, Trl);
     }
-    scan34_df(M, lane, min(32, N - s));
-    if (nw > 1) {
-      if (lane == 31) {
+    df m[4];
+    {
+      const df *T = buf[f];
 #pragma unroll
-        for (int q = 0; q < 12; ++q) tot[warp][q] = M[q];
-      }
-      __syncthreads();
-      if (warp == 0) {  // lane w < nw: the carry and the products of the warps before w; lane nw: the next carry
-        df E[12];
+      for (int j = 0; j < 3; ++j) m[j] = T[4 * j + r];
+      m[3] = -df_dot3(m[0].h, m[0].l, m[1].h, m[1].l, m[2].h, m[2].l, T[3], T[7], T[11]);
+    }
+    __syncthreads();
 #pragma unroll
-        for (int q = 0; q < 12; ++q) E[q] = lane == 0 || lane > nw ? carry[q] : tot[lane - 1][q];
-        scan34_df(E, lane, nw + 1);
-        __syncwarp();
-        if (lane < nw) {
+    for (int j = 0; j < 4; ++j) buf[f][4 * r + j] = m[j];
+    __syncthreads();
+    // inclusive scan: M_k <- M_0 M_1 ... M_k (earlier factors on the left)
+    for (int d = 1; d < n; d <<= 1) {
+      const bool on = f >= d && f < n;
+      if (on) {
+        df p[4];
 #pragma unroll
-          for (int q = 0; q < 12; ++q) tot[lane][q] = E[q];
-        } else if (lane == nw) {
-#pragma unroll
-          for (int q = 0; q < 12; ++q) carry_s[q] = E[q];
-        }
+        for (int j = 0; j < 4; ++j) p[j] = buf[f - d][4 * r + j];
+        compose_row_df(p, buf[f], m);
       }
       __syncthreads();
+      if (on) {
 #pragma unroll
-      for (int q = 0; q < 12; ++q) carry[q] = tot[warp][q];
+        for (int j = 0; j < 4; ++j) buf[f][4 * r + j] = m[j];
+      }
+      __syncthreads();
     }
-    if (k < N) {
-      df G[12];
-      compose34_df(carry, M, G);
-      write_frame_df(wv, (size_t)(fo + k + 1), G, Trl);
-    }
-    if (nw > 1) {
+    if (s > 0 && k < N) {
+      df p[4];
 #pragma unroll
-      for (int q = 0; q < 12; ++q) carry[q] = carry_s[q];
-      __syncthreads();  // (the next pass writes tot and carry_s)
-    } else if (s + 32 < N) {
-      df G[12];
-      compose34_df(carry, M, G);
-#pragma unroll
-      for (int q = 0; q < 12; ++q) carry[q] = df{__shfl_sync(0xffffffffu, G[q].h, 31), __shfl_sync(0xffffffffu, G[q].l, 31)};
+      for (int j = 0; j < 4; ++j) p[j] = last[4 * r + j];
+      compose_row_df(p, buf[f], m);
     }
+    if (k < N) write_frame_row_df(wv, (size_t)(fo + k + 1), r, m, Trl);
+    if (s + nf >= N) break;
+    __syncthreads();  // (every product with the carried prefix is formed)
+    if (f == nf - 1) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) last[4 * r + j] = m[j];
+    }
+    __syncthreads();
   }
 }
 
@@ -462,8 +424,8 @@ int launch_chain(const PlanView &pv, const WorkView &wv, const double *poses, in
     k_chain<<<pv.B, 96 * std::min(kChainFrames / 32, std::max(1, (pv.max_P / 6 + 31) / 32)), 0, (cudaStream_t)stream>>>(
         pv, wv, poses, gate);
   else
-    k_chain_df<<<pv.B, 32 * std::min(kChainWarps, std::max(1, (pv.max_P / 6 + 31) / 32)), 0, (cudaStream_t)stream>>>(
-        pv, wv, poses, gate);
+    k_chain_df<<<pv.B, 96 * std::min(kChainDfFrames / 32, std::max(1, (pv.max_P / 6 + 31) / 32)), 0,
+                 (cudaStream_t)stream>>>(pv, wv, poses, gate);
   ++g_launches;
   return (int)cudaGetLastError();
 }

@@ -659,23 +659,26 @@ int launch_backsub(const PlanView &pv, const WorkView &wv, const Params &prm, co
 }
 
 // ---- T_k <- T_k Exp(scale * delta_k) in FP64; pred += delta^T (g + lam diag(A) delta) ----
-// gacc: the accurate pose gradient of the refined step (else g of the linearisation)
+// gacc: the accurate pose gradient of the refined step (else g of the linearisation).
+// Four lanes per pose: lane r < 3 forms row r of the new pose and two terms of pred.  Bound by the
+// FP64 instructions and conversions of one warp (64 cycles each): a thread per pose 8.2 us for a
+// 10-pose window, 5.1 us so.
 template <typename T>
 __global__ void k_update_poses(PlanView pv, WorkView wv, const double *poses, double *out, double scale,
                                int gate, const double *gacc) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, p = t >> 2, r = t & 3;
   if (p >= pv.NP) return;
   const int b = pv.pose_prob[p];
   if (!problem_active(wv.lm, b, gate)) return;
   const int k = p - pv.p_pose_off[b];
   const int P = 6 * pv.p_npose[b];
   const int po = pv.p_param_off[b] + 6 * k;
-  double xi[6], T0[12];
+  double xi[6], T0[4];  // row r (lane 3: row 2 again, dropped)
 #pragma unroll
   for (int q = 0; q < 6; ++q) xi[q] = scale * wv.delta[po + q];
 #pragma unroll
-  for (int q = 0; q < 12; ++q) T0[q] = poses[12 * (size_t)p + q];
-  double Tn[12];
+  for (int q = 0; q < 4; ++q) T0[q] = poses[12 * (size_t)p + 4 * min(r, 2) + q];
+  double Tn[4];
   if constexpr (std::is_same<T, float>::value) {
     // FP32 path: T_new = T + T (Exp(xi) - I), the increment Exp(xi) - I formed in FP32
     // (relative precision of the increment itself) and the sum in double-float, so
@@ -714,45 +717,48 @@ __global__ void k_update_poses(PlanView pv, WorkView wv, const double *poses, do
       const float jz = (i == 2 ? 1.f : 0.f) + b * S[3 * i + 2] + c * S2[3 * i + 2];
       D[4 * i + 3] = jx * rx + jy * ry + jz * rz;
     }
-    df Rd[9];
+    df Td[4];
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 4; ++j) Td[j] = df_from_double(T0[j]);
 #pragma unroll
-      for (int j = 0; j < 3; ++j) Rd[3 * i + j] = df_from_double(T0[4 * i + j]);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        // (T D)(i, j) = sum_k R(i, k) D(k, j)  (D's last row is zero)
-        const df td = Rd[3 * i] * D[j] + Rd[3 * i + 1] * D[4 + j] + Rd[3 * i + 2] * D[8 + j];
-        const df v = df_from_double(T0[4 * i + j]) + td;
-        Tn[4 * i + j] = (double)v.h + (double)v.l;
-      }
+    for (int j = 0; j < 4; ++j) {
+      // (T D)(r, j) = sum_k R(r, k) D(k, j)  (D's last row is zero)
+      const df v = Td[j] + (Td[0] * D[j] + Td[1] * D[4 + j] + Td[2] * D[8 + j]);
+      Tn[j] = (double)v.h + (double)v.l;
     }
   } else {
     double E[12];
     exp_se3(xi, E);
-    compose34(T0, E, Tn);
-  }
 #pragma unroll
-  for (int q = 0; q < 12; ++q) out[12 * (size_t)p + q] = Tn[q];
+    for (int j = 0; j < 4; ++j) Tn[j] = T0[0] * E[j] + T0[1] * E[4 + j] + T0[2] * E[8 + j];
+    Tn[3] += T0[3];
+  }
+  if (r < 3) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) out[12 * (size_t)p + 4 * r + q] = Tn[q];
+  }
   const double lam = wv.lm[b].lam;
   const T *A = reinterpret_cast<const T *>(wv.A) + pv.p_S_off[b];
   const T *g = reinterpret_cast<const T *>(wv.g);
   double pred = 0.0;
 #pragma unroll
-  for (int q = 0; q < 6; ++q) {
+  for (int h = 0; h < 2; ++h) {
+    const int q = 2 * min(r, 2) + h;
     const double d = wv.delta[po + q];
     const double akk = (double)A[(size_t)(6 * k + q) * P + 6 * k + q];
     pred += d * ((gacc ? gacc[po + q] : (double)g[po + q]) + lam * akk * d);
   }
-  atomicAdd(wv.pred_acc + b, pred);
+  if (r == 3) pred = 0.0;
+  const unsigned four = 0xfu << (threadIdx.x & 28);
+  pred += __shfl_xor_sync(four, pred, 1);
+  pred += __shfl_xor_sync(four, pred, 2);
+  if (r == 0) atomicAdd(wv.pred_acc + b, pred);
 }
 
 template <typename T>
 int launch_update_poses(const PlanView &pv, const WorkView &wv, const double *poses, double *poses_out,
                         double scale, int direct, void *stream, const double *gacc) {
-  k_update_poses<T><<<grid_for(pv.NP, 128), 128, 0, (cudaStream_t)stream>>>(pv, wv, poses, poses_out, scale,
+  k_update_poses<T><<<grid_for(4ll * pv.NP, 128), 128, 0, (cudaStream_t)stream>>>(pv, wv, poses, poses_out, scale,
                                                                        direct ? GATE_ALL : GATE_RUNNING, gacc);
   ++g_launches;
   return (int)cudaGetLastError();

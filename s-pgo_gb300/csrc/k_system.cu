@@ -184,33 +184,70 @@ __device__ __forceinline__ void df_rel_c(const WorkView &wv, int fx, int fy, df 
            df_make(wv.fr_cl[(size_t)fx * 6 + k] - wv.fr_cl[(size_t)fy * 6 + k]);
 }
 
-constexpr int kPrThreads = 512;
+constexpr int kPrThreads = 896;  // thread per (pose, component) of a 33-pose window
 
 // 0. every record (lo, hi): read (FP64) and cleared, split into double-float, moved from
-// c_lo to o; one thread per record
+// c_lo to o.  A CTA stages kShRecs records in shared memory (whole lines in and out); lane i of
+// three moves row i of a record's P and Q (shift_record's formulas; row i of Z R, Q Z and (Z R) Z
+// and column i of Q Z).  Bound by the latency of one record's double-float chain: a thread per
+// record 11.4 us for a 10-pose window and 19.3 us for 64 of up to 32 poses, 7.2 and 11.2 us so.
+constexpr int kShRecs = 32;
+
 __global__ void __launch_bounds__(128) k_pair_shift_df(PlanView pv, WorkView wv) {
   const int b = blockIdx.y;
   if (!problem_active(wv.lm, b, GATE_RELIN)) return;
-  const int N = pv.p_npose[b], D = pv.p_pair_D[b];
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= N * D) return;
-  const int lo = r / D, hi = lo + r % D + 1;
-  if (hi > N) return;
-  const int fo = pv.p_frame_off[b];
-  double *rec = reinterpret_cast<double *>(wv.pair_acc) + ((size_t)pv.p_pair_off[b] + r) * 27;
-  df v[27];
-#pragma unroll
-  for (int k = 0; k < 27; ++k) v[k] = df_split_double(rec[k]);
-#pragma unroll
-  for (int k = 0; k < 27; ++k) rec[k] = 0.0;  // cleared for the next linearisation
-  if (lo > 0) {
-    df z[3];
-    df_rel_c(wv, fo + lo, fo, z);  // from c_lo to o = c_0
-    shift_record(v, z);
+  __shared__ df v[kShRecs * 27];
+  const int N = pv.p_npose[b], D = pv.p_pair_D[b], fo = pv.p_frame_off[b];
+  const int r0 = blockIdx.x * kShRecs, n = min(kShRecs, N * D - r0);
+  if (n <= 0) return;
+  const size_t off = ((size_t)pv.p_pair_off[b] + r0) * 27;
+  double *rec = reinterpret_cast<double *>(wv.pair_acc) + off;
+  df *out = reinterpret_cast<df *>(wv.pairF) + off;
+  auto valid = [&](int r) { return (r0 + r) / D + (r0 + r) % D + 1 <= N; };
+  for (int q = threadIdx.x; q < 27 * n; q += blockDim.x) {
+    if (!valid(q / 27)) continue;
+    v[q] = df_split_double(rec[q]);
+    rec[q] = 0.0;  // cleared for the next linearisation
   }
-  df *out = reinterpret_cast<df *>(wv.pairF) + ((size_t)pv.p_pair_off[b] + r) * 27;
+  __syncthreads();
+  const int r = threadIdx.x >> 2, i = threadIdx.x & 3, lo = (r0 + r) / D;
+  const bool mine = r < n && i < 3 && lo > 0 && valid(r);
+  df p[3], q[3], mw;
+  if (mine) {
+    const df *m = v + 27 * r;
+    const int i1 = i == 2 ? 0 : i + 1, i2 = i == 0 ? 2 : i - 1;
+    df z[3], qi[3];
+    df_rel_c(wv, fo + lo, fo, z);  // from c_lo to o = c_0
+    const df z1 = i == 0 ? z[1] : i == 1 ? z[2] : z[0], z2 = i == 0 ? z[2] : i == 1 ? z[0] : z[1];
+    df zr[3], qz[3], zrz[3];
 #pragma unroll
-  for (int k = 0; k < 27; ++k) out[k] = v[k];
+    for (int j = 0; j < 3; ++j) {
+      qi[j] = m[t6(i, 3 + j)];
+      zr[j] = z1 * m[t6(3 + i2, 3 + j)] - z2 * m[t6(3 + i1, 3 + j)];
+    }
+    cross3(z, qi, qz);   // -(Q Z)[i, :]
+    cross3(z, zr, zrz);  // -((Z R) Z)[i, :]
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const df qzc = z1 * m[t6(c, 3 + i2)] - z2 * m[t6(c, 3 + i1)];  // -(Q Z)[c, i]
+      p[c] = m[t6(i, c)] + qz[c] + qzc + zrz[c];
+      q[c] = qi[c] + zr[c];
+    }
+    mw = m[21 + i] + (z1 * m[24 + i2] - z2 * m[24 + i1]);
+  }
+  __syncthreads();
+  if (mine) {
+    df *m = v + 27 * r;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      if (c >= i) m[t6(i, c)] = p[c];
+      m[t6(i, 3 + c)] = q[c];
+    }
+    m[21 + i] = mw;
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < 27 * n; k += blockDim.x)
+    if (valid(k / 27)) out[k] = v[k];
 }
 
 // 1. thread per (hi, component): prefix over lo, P(i, hi) = sum_{lo <= i} M(lo, hi);
@@ -377,9 +414,9 @@ int launch_system(const PlanView &pv, const WorkView &wv, int gate, void *stream
   const int nmax = pv.max_P / 6;
   const int nd = pv.max_D > 0 ? pv.max_D : 1;
   if constexpr (std::is_same<T, float>::value) {
-    k_pair_shift_df<<<dim3(grid_for((long long)nmax * nd, 128), pv.B), 128, 0, st>>>(pv, wv);
+    k_pair_shift_df<<<dim3(grid_for((long long)nmax * nd, kShRecs), pv.B), 4 * kShRecs, 0, st>>>(pv, wv);
     if (nmax <= kPrWide) {
-      k_pair_scan_df<0><<<pv.B, kPrThreads, 0, st>>>(pv, wv);
+      k_pair_scan_df<0><<<pv.B, std::min(kPrThreads, 32 * grid_for(27 * nmax, 32)), 0, st>>>(pv, wv);
     } else {
       const dim3 grid(pv.B, grid_for((long long)nmax * 27, 128));
       k_pair_scan_df<1><<<grid, 128, 0, st>>>(pv, wv);
