@@ -162,6 +162,8 @@ struct spgo_plan {
   std::vector<int32_t> tc_prob, tc_row0, tc_col0, tc_ncols, tc_cbeg, tc_cend, tc_chunks;
   // batched factorisation: CTA k factors problem fs_prob[k], widest first
   std::vector<int32_t> fs_prob;
+  // passes over the observations: CTA k takes chunk ch_sched[k].x of problem ch_sched[k].y
+  std::vector<int2> ch_sched;
   std::vector<Seg> segs;
   size_t static_bytes = 0, ws_bytes = 0;
   // host staging: [0, big_bytes) of the device buffer, then the small arrays
@@ -263,6 +265,7 @@ static void build_layout(spgo_plan *p) {
   small(p->tc_prob); small(p->tc_row0); small(p->tc_col0); small(p->tc_ncols);
   small(p->tc_cbeg); small(p->tc_cend); small(p->tc_chunks);
   small(p->fs_prob);
+  small(p->ch_sched);
   p->small = arena_get(p->static_bytes - p->big_bytes);
   for (size_t i = 0; i < p->segs.size(); ++i)
     if (small_src[i] && p->segs[i].bytes)
@@ -653,6 +656,14 @@ static int plan_build(const spgo_host_problem *probs, int nprob, int precision, 
     std::stable_sort(p->fs_prob.begin(), p->fs_prob.end(),
                      [&](int32_t x, int32_t y) { return p->p_npose[x] > p->p_npose[y]; });
   }
+  {  // most observations first: a chunk of a wide window takes up to ten times as long as one of a
+     // narrow window, and a long one that starts last leaves the GPU to itself
+    const auto obs = [&](int32_t c) { return p->lm_obs[p->ch_lm0[c] + p->ch_cnt[c]] - p->lm_obs[p->ch_lm0[c]]; };
+    p->ch_sched.resize(p->ch_prob.size());
+    for (size_t c = 0; c < p->ch_sched.size(); ++c) p->ch_sched[c] = make_int2((int)c, p->ch_prob[c]);
+    std::stable_sort(p->ch_sched.begin(), p->ch_sched.end(),
+                     [&](const int2 &x, const int2 &y) { return obs(x.x) > obs(y.x); });
+  }
   build_layout(p);
   return SPGO_OK;
 }
@@ -767,6 +778,7 @@ static void make_views(spgo_solver *s) {
   v.tc_cbeg = seg_ptr<int32_t>(p, st, i++); v.tc_cend = seg_ptr<int32_t>(p, st, i++);
   v.tc_chunks = seg_ptr<int32_t>(p, st, i++);
   v.fs_prob = seg_ptr<int32_t>(p, st, i++);
+  v.ch_sched = seg_ptr<int2>(p, st, i++);
   v.n_tc_items = (int32_t)p->tc_prob.size();
   v.n_tc_chunks = (int32_t)p->tc_chunks.size();
   for (size_t k = 0; k < p->wk_prob.size(); ++k) v.wk_max_len = std::max(v.wk_max_len, p->wk_cend[k] - p->wk_cbeg[k]);

@@ -122,8 +122,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_jacobian(PlanVi
   constexpr bool kMixed = std::is_same<T, float>::value;
   constexpr int kRow = kJacRow<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int c = blockIdx.x;
-  const int b = pv.ch_prob[c];
+  const int2 cb = pv.ch_sched[blockIdx.x];
+  const int c = cb.x, b = cb.y;
   if (!problem_active(wv.lm, b, gate)) return;
   const int tid = threadIdx.x, lane = tid & 31;
   const int f0 = pv.ch_f0[c], nb = pv.ch_nb[c], lm0 = pv.ch_lm0[c], cnt = pv.ch_cnt[c];

@@ -187,8 +187,8 @@ __global__ void __launch_bounds__(kRpThreads, 8) k_resid_pass(PlanView pv, WorkV
                                                            const double *__restrict__ alpha_state) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ RefSmem sm;
-  const int c = blockIdx.x;
-  const int b = pv.ch_prob[c];
+  const int2 cb = pv.ch_sched[blockIdx.x];
+  const int c = cb.x, b = cb.y;
   if (!refine_active(wv, b)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int f0 = pv.ch_f0[c], nb = pv.ch_nb[c], lm0 = pv.ch_lm0[c], cnt = pv.ch_cnt[c];

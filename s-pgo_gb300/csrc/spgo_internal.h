@@ -55,6 +55,8 @@ struct PlanView {                 // device pointers into the static buffer
   // chunks
   const int32_t *ch_prob, *ch_f0, *ch_nb, *ch_lm0, *ch_cnt;
   const int64_t *ch_slab;
+  // (chunk, problem) per CTA of the passes over the observations, most observations first
+  const int2 *ch_sched;
   // Schur work items
   const int32_t *wk_prob, *wk_ti, *wk_tj, *wk_cbeg, *wk_cend, *wk_chunks;
   // frame -> problem
