@@ -552,7 +552,9 @@ class CudaSolver:
         T = np.asarray(T_curr_to_next_py, dtype=np.float32).reshape(4, 4)
         self._sync_from_device()
         self._poses[k, :3, :] = T[:3, :]
-        self._push_state()
+        if self._solver is not None:
+            row = self._solver.poses[:12 * self._N].view(self._N, 12)[k]
+            row.copy_(torch.from_numpy(self._poses[k, :3, :].reshape(-1)))
 
     def getIncrementalPose(self, keyFrameID):
         self._sync_from_device()
@@ -561,7 +563,8 @@ class CudaSolver:
     def loadInverseDepths(self, inverse_depths_py):
         self._sync_from_device()
         self._alpha = np.asarray(inverse_depths_py, dtype=np.float32).reshape(-1).astype(np.float64)
-        self._push_state()
+        if self._solver is not None:
+            self._solver.set_alpha(0, self._alpha[self._feats])
 
     def getInverseDepths(self):
         self._sync_from_device()
@@ -577,17 +580,19 @@ class CudaSolver:
             self._build()
         if self._solver is None:
             return
-        self._solver.gn_step(int(iterations), self._step_size)
         self._on_device = True
+        self._solver.gn_step(int(iterations), self._step_size)
         # features without measurements still have their inverse depth clamped (Solver_cuda.cu:545-546)
         if int(iterations) > 0:
-            rest = np.ones(self._alpha.size, dtype=bool)
-            rest[self._feats] = False
-            self._alpha[rest] = np.clip(self._alpha[rest], 1.0 / 30.0, 1.0 / 0.2)
+            if self._rest is None or self._rest.size != self._alpha.size:
+                self._rest = np.ones(self._alpha.size, dtype=bool)
+                self._rest[self._feats] = False
+            self._alpha[self._rest] = np.clip(self._alpha[self._rest], 1.0 / 30.0, 1.0 / 0.2)
         self._solver.synchronize()
 
     # --- internals ------------------------------------------------------------------------
-    _on_device = False
+    _on_device = False   # the device holds a newer state than the host copies (after a step)
+    _rest: Optional[np.ndarray] = None  # features without measurements
 
     def _problem(self) -> Optional[Problem]:
         L = self._N * self._M
@@ -600,6 +605,7 @@ class CudaSolver:
             targets.setdefault(f, set()).add(t)
         feats = sorted(anchors)
         self._feats = np.array(feats, dtype=np.int64)
+        self._rest = None
         if not feats:
             return None
         host = np.array([anchors[f] for f in feats], dtype=np.int32)
@@ -633,7 +639,7 @@ class CudaSolver:
         self._solver.set_params(loss="cauchy", loss_scale=3.0, near_boost=True, eps=1e-4,
                                 alpha_min=1.0 / 30.0, alpha_max=1.0 / 0.2)
         self._dirty = False
-        self._on_device = True
+        self._on_device = False
 
     def _sync_from_device(self):
         if self._solver is not None and self._on_device:
@@ -641,9 +647,3 @@ class CudaSolver:
             a = self._solver.get_alpha(0)
             self._alpha[self._feats] = a
             self._on_device = False
-
-    def _push_state(self):
-        if self._solver is not None:
-            self._solver.set_poses(0, self._poses)
-            self._solver.set_alpha(0, self._alpha[self._feats])
-            self._on_device = True
