@@ -245,6 +245,7 @@ __device__ __forceinline__ void bd_invert_diag(const float *B, const float *rinv
 // one CTA per block column of each end.  sx: also the exact S (hi, lo), both triangles, for
 // the residual of the reduced solve's own refinement.
 __global__ void __launch_bounds__(256) k_band_assemble(PlanView pv, WorkView wv, int b, int sx) {
+  grid_enter();
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   const BandGeo geo(pv.p_npose[b], pv.p_pair_D[b]);
   const int e = (int)blockIdx.x >= geo.mR, c = (int)blockIdx.x - geo.base(e);
@@ -293,6 +294,7 @@ __global__ void __launch_bounds__(256) k_band_assemble(PlanView pv, WorkView wv,
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBandThreads) k_band_factor(PlanView pv, WorkView wv, int b,
                                                                                         uint64_t wait_ns) {
+  grid_enter();
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   extern __shared__ __align__(16) float blocks[];
   __shared__ float rinv[2][kBb];
@@ -462,6 +464,7 @@ __device__ __forceinline__ int bd_at(int c, int i) { return c * kBb + 4 * ((i >>
 // (thread = (block further away, unknown)) apply the block before it.
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBandSolveThreads)
     k_band_solve(PlanView pv, WorkView wv, int b, int first, int last, int accum, uint64_t wait_ns) {
+  grid_enter();
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   extern __shared__ __align__(16) float stage[];               // [kBandStages][h + 1][kBandBlk]
   __shared__ __align__(16) float ring[(SPGO_BAND_MAX_H + 2) * kBb];  // running right-hand sides, then solutions

@@ -53,6 +53,7 @@ template <> struct ExactS<double> { using type = double; };
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_lg_assemble(PlanView pv, WorkView wv, int b) {
+  grid_enter();
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   const int P = 6 * pv.p_npose[b], r = blockIdx.x;
   if (r >= P) return;
@@ -104,6 +105,7 @@ __global__ void __launch_bounds__(256) k_lg_assemble(PlanView pv, WorkView wv, i
 // The diagonal block is kept as U, which the substitutions read, and 1 / L(k, k); U goes to the
 // transposed place (the upper triangle: other CTAs may still read S_kk).
 __global__ void __launch_bounds__(32 * kLgPanelRows) k_lg_panel(PlanView pv, WorkView wv, int b, int kb) {
+  grid_enter();
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   constexpr int NB = LgShape<double>::NB, W = kLgPanelRows, C = NB / W;
   static_assert(NB == 32, "lane = row of the diagonal block");
@@ -169,6 +171,7 @@ __device__ __forceinline__ T lg_diag(const T *L, const T *dinv, int P, int i, in
 // the shared column times 1 / L(k, k).  The serial part per column is one barrier,
 // one square root and one reciprocal; the update is spread over the rows.
 __global__ void __launch_bounds__(kLgNB) k_lg_potrf_rows(PlanView pv, WorkView wv, int b, int kb) {
+  grid_enter();
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   __shared__ float col[2][kLgNB];
   const int P = 6 * pv.p_npose[b], nb = min(kLgNB, P - kb), i = threadIdx.x;
@@ -213,6 +216,7 @@ __global__ void __launch_bounds__(kLgNB) k_lg_potrf_rows(PlanView pv, WorkView w
 // (once x_j is final it is removed from every later column: independent updates
 // instead of one dependent chain per column)
 __global__ void __launch_bounds__(128) k_lg_trsm(PlanView pv, WorkView wv, int b, int kb) {
+  grid_enter();
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   __shared__ float D[kLgNB][kLgNB + 1];
   __shared__ float di[kLgNB];
@@ -255,6 +259,7 @@ __global__ void __launch_bounds__(128) k_lg_trsm(PlanView pv, WorkView wv, int b
 // (the next panel's columns), mode 2 the others
 template <typename T>
 __global__ void __launch_bounds__(256) k_lg_syrk(PlanView pv, WorkView wv, int b, int kb, int mode) {
+  grid_enter();
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   constexpr int NB = LgShape<T>::NB, TS = LgShape<T>::TS, R = TS / 16;
   __shared__ T LR[NB][TS + 1];
@@ -339,6 +344,7 @@ __device__ __forceinline__ void lg_set_flag(int *flag) {
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_lg_fwd(PlanView pv, WorkView wv, int b, int first, uint64_t wait_ns) {
+  grid_enter();
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   __shared__ T part[4][kLgNB];
   __shared__ T zs[kLgNB];
@@ -431,6 +437,7 @@ __global__ void __launch_bounds__(256) k_lg_fwd(PlanView pv, WorkView wv, int b,
 template <typename T>
 __global__ void __launch_bounds__(256) k_lg_bwd(PlanView pv, WorkView wv, int b, int first, int last, int accum,
                                                  uint64_t wait_ns) {
+  grid_enter();
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   __shared__ T part[4][kLgNB];
   __shared__ T zs[kLgNB];
@@ -542,6 +549,7 @@ __global__ void __launch_bounds__(256) k_lg_bwd(PlanView pv, WorkView wv, int b,
 // assembly cleared S_L inside the band only; what a non-finite 1 / D may have spread beyond
 // it (such an S always fails the factor) goes here.
 __global__ void k_lg_zero_failed(PlanView pv, WorkView wv, int b, int band) {
+  grid_enter();
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   if (!wv.lm[b].fail) return;
   const int P = 6 * pv.p_npose[b], po = pv.p_param_off[b];
@@ -555,6 +563,7 @@ __global__ void k_lg_zero_failed(PlanView pv, WorkView wv, int b, int band) {
 // residual y = g0 - S x from the exact S, warp per row
 template <typename T>
 __global__ void __launch_bounds__(256) k_lg_resid(PlanView pv, WorkView wv, int b) {
+  grid_enter();
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   const int P = 6 * pv.p_npose[b], po = pv.p_param_off[b];
   const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -592,18 +601,20 @@ int launch_factor_large(const PlanView &pv, const WorkView &wv, const Params &pr
     int rc = launch_band_factor(pv, wv, prm, b, N, D, refine > 0, stream);
     for (int it = 0; rc == 0 && it <= refine; ++it) {
       if (it > 0) {
-        k_lg_resid<T><<<(P + 7) / 8, 256, 0, st>>>(pv, wv, b);
+        launch(k_lg_resid<T>, (P + 7) / 8, 256, 0, st, pv, wv, b);
         ++g_launches;
       }
       rc = launch_band_solve(pv, wv, prm, b, N, D, it == 0, it == refine, 0, stream);
     }
-    k_lg_zero_failed<<<grid_for(P, 256), 256, 0, st>>>(pv, wv, b, 1);
+    launch(k_lg_zero_failed, grid_for(P, 256), 256, 0, st, pv, wv, b, 1);
     ++g_launches;
     return rc ? rc : (int)cudaGetLastError();
   }
   const uint64_t wait_ns = wait_limit_ns(prm);
-  k_lg_assemble<T><<<P, 256, 0, st>>>(pv, wv, b);
+  launch(k_lg_assemble<T>, P, 256, 0, st, pv, wv, b);
   int n = 1;
+  // (the panels' kernels are launched plainly: CTAs that come in while the kernel before still
+  // fills most SMs share the others', and a 600-wide FP64 system took 1.74 ms instead of 1.64)
   constexpr int NB = LgShape<T>::NB, TS = LgShape<T>::TS;
   const int bw = 6 * D - 1;  // S and L are zero beyond it: a panel reaches bw rows down
   if constexpr (std::is_same<T, double>::value) {
@@ -652,18 +663,18 @@ int launch_factor_large(const PlanView &pv, const WorkView &wv, const Params &pr
   int *ff = wv.lg_flag + param_off, *fb = wv.lg_flag + pv.total_params + param_off;
   for (int it = 0; it <= refine; ++it) {
     if (it > 0) {
-      k_lg_resid<T><<<(P + 7) / 8, 256, 0, st>>>(pv, wv, b);
+      launch(k_lg_resid<T>, (P + 7) / 8, 256, 0, st, pv, wv, b);
       ++n;
     }
     cudaError_t e = cudaMemsetAsync(ff, 0, sizeof(int) * (size_t)nblk, st);
     if (e != cudaSuccess) return (int)e;
-    k_lg_fwd<T><<<nblk, 256, 0, st>>>(pv, wv, b, it == 0, wait_ns);
+    launch(k_lg_fwd<T>, nblk, 256, 0, st, pv, wv, b, it == 0, wait_ns);
     e = cudaMemsetAsync(fb, 0, sizeof(int) * (size_t)nblk, st);
     if (e != cudaSuccess) return (int)e;
-    k_lg_bwd<T><<<nblk, 256, 0, st>>>(pv, wv, b, it == 0, it == refine, 0, wait_ns);
+    launch(k_lg_bwd<T>, nblk, 256, 0, st, pv, wv, b, it == 0, it == refine, 0, wait_ns);
     n += 2;
   }
-  k_lg_zero_failed<<<grid_for(P, 256), 256, 0, st>>>(pv, wv, b, 0);
+  launch(k_lg_zero_failed, grid_for(P, 256), 256, 0, st, pv, wv, b, 0);
   ++n;
   g_launches += n;
   return (int)cudaGetLastError();
@@ -681,10 +692,10 @@ int launch_refine_large(const PlanView &pv, const WorkView &wv, const Params &pr
   int *ff = wv.lg_flag + param_off, *fb = wv.lg_flag + pv.total_params + param_off;
   cudaError_t e = cudaMemsetAsync(ff, 0, sizeof(int) * (size_t)nblk, st);
   if (e != cudaSuccess) return (int)e;
-  k_lg_fwd<float><<<nblk, 256, 0, st>>>(pv, wv, b, 0, wait_ns);
+  launch(k_lg_fwd<float>, nblk, 256, 0, st, pv, wv, b, 0, wait_ns);
   e = cudaMemsetAsync(fb, 0, sizeof(int) * (size_t)nblk, st);
   if (e != cudaSuccess) return (int)e;
-  k_lg_bwd<float><<<nblk, 256, 0, st>>>(pv, wv, b, 0, 0, 1, wait_ns);
+  launch(k_lg_bwd<float>, nblk, 256, 0, st, pv, wv, b, 0, 0, 1, wait_ns);
   g_launches += 2;
   return (int)cudaGetLastError();
 }

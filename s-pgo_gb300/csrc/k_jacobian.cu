@@ -117,6 +117,7 @@ template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_jacobian(PlanView pv, WorkView wv, Params prm,
                                                                          const double *__restrict__ alpha_state,
                                                                          int gate) {
+  grid_enter();
   using M = Num<T>;
   using V = typename M::V;
   constexpr bool kMixed = std::is_same<T, float>::value;
@@ -429,7 +430,7 @@ int launch_jacobian(const PlanView &pv, const WorkView &wv, const Params &prm, c
   cudaFuncSetAttribute(k_jacobian<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   // all of the unified L1 / shared memory as shared: the resident CTAs fill it
   cudaFuncSetAttribute(k_jacobian<T>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-  k_jacobian<T><<<pv.n_chunks, nt, sm, (cudaStream_t)stream>>>(pv, wv, prm, alpha, gate);
+  launch(k_jacobian<T>, pv.n_chunks, nt, sm, (cudaStream_t)stream, pv, wv, prm, alpha, gate);
   ++g_launches;
   return (int)cudaGetLastError();
 }

@@ -74,6 +74,7 @@ __device__ __forceinline__ void compose_row(const double *p, const double *M, do
 
 __global__ void __launch_bounds__(3 * kChainFrames) k_chain(PlanView pv, WorkView wv, const double *__restrict__ poses,
                                                             int gate) {
+  grid_enter();
   const int b = blockIdx.x;
   if (!problem_active(wv.lm, b, gate)) return;
   __shared__ double buf[2][kChainFrames][12];
@@ -156,6 +157,7 @@ __host__ __device__ inline size_t cost_smem(int max_nb, size_t *dc) {
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_cost(PlanView pv, WorkView wv, Params prm,
                                                    const double *__restrict__ alpha_state, int gate) {
+  grid_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int2 cb = pv.ch_sched[blockIdx.x];
   const int c = cb.x, b = cb.y;
@@ -356,6 +358,7 @@ constexpr int kChainDfFrames = 256;
 
 __global__ void __launch_bounds__(3 * kChainDfFrames) k_chain_df(PlanView pv, WorkView wv,
                                                                  const double *__restrict__ poses, int gate) {
+  grid_enter();
   const int b = blockIdx.x;
   if (!problem_active(wv.lm, b, gate)) return;
   __shared__ df buf[kChainDfFrames][12];
@@ -421,11 +424,10 @@ __global__ void __launch_bounds__(3 * kChainDfFrames) k_chain_df(PlanView pv, Wo
 
 int launch_chain(const PlanView &pv, const WorkView &wv, const double *poses, int gate, int f64, void *stream) {
   if (f64)
-    k_chain<<<pv.B, 96 * std::min(kChainFrames / 32, std::max(1, (pv.max_P / 6 + 31) / 32)), 0, (cudaStream_t)stream>>>(
+    launch(k_chain, pv.B, 96 * std::min(kChainFrames / 32, std::max(1, (pv.max_P / 6 + 31) / 32)), 0, (cudaStream_t)stream, 
         pv, wv, poses, gate);
   else
-    k_chain_df<<<pv.B, 96 * std::min(kChainDfFrames / 32, std::max(1, (pv.max_P / 6 + 31) / 32)), 0,
-                 (cudaStream_t)stream>>>(pv, wv, poses, gate);
+    launch(k_chain_df, pv.B, 96 * std::min(kChainDfFrames / 32, std::max(1, (pv.max_P / 6 + 31) / 32)), 0, (cudaStream_t)stream, pv, wv, poses, gate);
   ++g_launches;
   return (int)cudaGetLastError();
 }
@@ -439,7 +441,7 @@ int launch_linearize(const PlanView &pv, const WorkView &wv, const Params &prm, 
   if (!cost_only) return launch_jacobian<T>(pv, wv, prm, alpha, gate, stream);
   const int nt = prm.cost_block > 0 ? prm.cost_block : kCostThreads;
   size_t dc;
-  k_cost<T><<<pv.n_chunks, nt, cost_smem<T>(pv.max_nb, &dc), (cudaStream_t)stream>>>(pv, wv, prm, alpha, gate);
+  launch(k_cost<T>, pv.n_chunks, nt, cost_smem<T>(pv.max_nb, &dc), (cudaStream_t)stream, pv, wv, prm, alpha, gate);
   ++g_launches;
   return (int)cudaGetLastError();
 }

@@ -77,6 +77,7 @@ constexpr int kTwThreads = 192;  // (six warps: one per component in the scan)
 constexpr int kTwSlice = 32;
 
 __global__ void __launch_bounds__(kTwThreads) k_pair_twists(PlanView pv, WorkView wv, int slice) {
+  grid_enter();
   __shared__ double tw_s[(kTwSlice + SPGO_MAX_WINDOW + 1) * 6];
   const int b = blockIdx.x, l0 = slice * blockIdx.y;
   const int N = pv.p_npose[b], D = pv.p_pair_D[b], fo = pv.p_frame_off[b], po = pv.p_param_off[b];
@@ -142,7 +143,7 @@ int launch_pair_twists(const PlanView &pv, const WorkView &wv, void *stream) {
   const int nmax = pv.max_P / 6;
   int slice = kTwSlice;
   while (slice > 8 && (long long)pv.B * ((nmax + slice - 1) / slice) < 152) slice /= 2;
-  k_pair_twists<<<dim3(pv.B, (nmax + slice - 1) / slice), kTwThreads, 0, (cudaStream_t)stream>>>(pv, wv, slice);
+  launch(k_pair_twists, dim3(pv.B, (nmax + slice - 1) / slice), kTwThreads, 0, (cudaStream_t)stream, pv, wv, slice);
   ++g_launches;
   return (int)cudaGetLastError();
 }
@@ -185,6 +186,7 @@ struct RpLayout {
 template <bool FIRST>
 __global__ void __launch_bounds__(kRpThreads, 8) k_resid_pass(PlanView pv, WorkView wv, Params prm,
                                                            const double *__restrict__ alpha_state) {
+  grid_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ RefSmem sm;
   const int2 cb = pv.ch_sched[blockIdx.x];
@@ -461,9 +463,9 @@ int launch_resid_pass(const PlanView &pv, const WorkView &wv, const Params &prm,
   cudaStream_t st = (cudaStream_t)stream;
   const size_t sm = RpLayout(pv.max_nb).total;
   if (first)
-    k_resid_pass<true><<<pv.n_chunks, kRpThreads, sm, st>>>(pv, wv, prm, alpha);
+    launch(k_resid_pass<true>, pv.n_chunks, kRpThreads, sm, st, pv, wv, prm, alpha);
   else
-    k_resid_pass<false><<<pv.n_chunks, kRpThreads, sm, st>>>(pv, wv, prm, alpha);
+    launch(k_resid_pass<false>, pv.n_chunks, kRpThreads, sm, st, pv, wv, prm, alpha);
   ++g_launches;
   return (int)cudaGetLastError();
 }
@@ -508,6 +510,7 @@ __device__ __forceinline__ void cp_async_wait_all() {
 }
 
 __global__ void __launch_bounds__(kRsThreads) k_resid_solve(PlanView pv, WorkView wv, float outer_tol) {
+  grid_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int b = pv.fs_prob[blockIdx.x];
   if (!refine_active(wv, b)) return;
@@ -659,6 +662,7 @@ __global__ void __launch_bounds__(kRsThreads) k_resid_solve(PlanView pv, WorkVie
 // order (FP64, segments of ~N / 42 poses).
 // (FP64-bound: small CTAs spread the sums over the SMs, and the centres come as FP64)
 __global__ void __launch_bounds__(64) k_rs_sums_large(PlanView pv, WorkView wv, int b) {
+  grid_enter();
   if (!refine_active(wv, b)) return;
   const int N = pv.p_npose[b], D = pv.p_pair_D[b], fo = pv.p_frame_off[b];
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -698,6 +702,7 @@ constexpr int kScanSegs = 42;  // segments per component: 6 x 42 = 252 of the 25
 
 // dynamic shared memory: the per-pose terms [N][6] (FP64)
 __global__ void __launch_bounds__(256) k_rs_scan_large(PlanView pv, WorkView wv, int b) {
+  grid_enter();
   if (!refine_active(wv, b)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double *val = reinterpret_cast<double *>(smem_raw);
@@ -745,6 +750,7 @@ __global__ void __launch_bounds__(256) k_rs_scan_large(PlanView pv, WorkView wv,
 }
 
 __global__ void __launch_bounds__(64) k_rs_rhs_large(PlanView pv, WorkView wv, int b) {
+  grid_enter();
   if (!refine_active(wv, b)) return;
   const int N = pv.p_npose[b], D = pv.p_pair_D[b], P = 6 * N;
   const int fo = pv.p_frame_off[b], po = pv.p_param_off[b];
@@ -781,11 +787,11 @@ __global__ void __launch_bounds__(64) k_rs_rhs_large(PlanView pv, WorkView wv, i
 int launch_resid_reduce_large(const PlanView &pv, const WorkView &wv, int b, int N, void *stream) {
   if (!wv.lg_red) return 0;  // (the FP64 path has no refinement)
   cudaStream_t st = (cudaStream_t)stream;
-  k_rs_sums_large<<<(12 * N + 63) / 64, 64, 0, st>>>(pv, wv, b);
+  launch(k_rs_sums_large, (12 * N + 63) / 64, 64, 0, st, pv, wv, b);
   const size_t sm = (size_t)N * 6 * sizeof(double);
   cudaFuncSetAttribute(k_rs_scan_large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_rs_scan_large<<<1, 256, sm, st>>>(pv, wv, b);
-  k_rs_rhs_large<<<std::max((N + 63) / 64, 96), 64, 0, st>>>(pv, wv, b);  // (the clearing wants the CTAs)
+  launch(k_rs_scan_large, 1, 256, sm, st, pv, wv, b);
+  launch(k_rs_rhs_large, std::max((N + 63) / 64, 96), 64, 0, st, pv, wv, b);  // (the clearing wants the CTAs)
   g_launches += 3;
   return (int)cudaGetLastError();
 }
@@ -795,7 +801,7 @@ int launch_resid_solve(const PlanView &pv, const WorkView &wv, const Params &prm
   const size_t sm = resid_solve_smem(pv.max_P_small, pv.max_P / 6);
   cudaStream_t st = (cudaStream_t)stream;
   cudaFuncSetAttribute(k_resid_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_resid_solve<<<pv.B, kRsThreads, sm, st>>>(pv, wv, prm.outer_steps > 1 ? prm.outer_tol : 0.f);
+  launch(k_resid_solve, pv.B, kRsThreads, sm, st, pv, wv, prm.outer_steps > 1 ? prm.outer_tol : 0.f);
   ++g_launches;
   return (int)cudaGetLastError();
 }
@@ -804,6 +810,7 @@ int launch_resid_solve(const PlanView &pv, const WorkView &wv, const Params &prm
 // one warp per chunk, lane = landmark slot: x_a += t - D^-1 W^T dx_p, alpha' =
 // clamp(alpha + x_a), pred += x_a (g_a + (lam C + eps) x_a) with the accurate g_a
 __global__ void k_backsub_refined(PlanView pv, WorkView wv, Params prm, const double *alpha, double *alpha_out) {
+  grid_enter();
   const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int slot = threadIdx.x & 31;
   if (c >= pv.n_chunks) return;
@@ -849,7 +856,7 @@ __global__ void k_backsub_refined(PlanView pv, WorkView wv, Params prm, const do
 int launch_backsub_refined(const PlanView &pv, const WorkView &wv, const Params &prm, const double *alpha,
                            double *alpha_out, void *stream) {
   if (pv.n_chunks == 0) return 0;
-  k_backsub_refined<<<grid_for(pv.n_chunks, 4), 128, 0, (cudaStream_t)stream>>>(pv, wv, prm, alpha, alpha_out);
+  launch(k_backsub_refined, grid_for(pv.n_chunks, 4), 128, 0, (cudaStream_t)stream, pv, wv, prm, alpha, alpha_out);
   ++g_launches;
   return (int)cudaGetLastError();
 }

@@ -109,6 +109,7 @@ __device__ __forceinline__ float split_row(const float *src, bool valid, const f
 
 
 __global__ void __launch_bounds__(kTcThreads, 1) k_schur_tc(PlanView pv, WorkView wv, Params prm, int gate) {
+  grid_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char *base = smem_raw + ((1024 - (tc::smem_u32(smem_raw) & 1023)) & 1023);
   TcSmem &sm = *reinterpret_cast<TcSmem *>(base);
@@ -364,7 +365,7 @@ int launch_schur_tc(const PlanView &pv, const WorkView &wv, const Params &prm, v
   if (pv.n_tc_items > 0) {
     const size_t sm = tc_smem_bytes();
     cudaFuncSetAttribute(k_schur_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_schur_tc<<<dim3(pv.n_tc_items, tc_shares(pv)), kTcThreads, sm, st>>>(pv, wv, prm, GATE_RUNNING);
+    launch(k_schur_tc, dim3(pv.n_tc_items, tc_shares(pv)), kTcThreads, sm, st, pv, wv, prm, GATE_RUNNING);
     ++g_launches;
   }
   return (int)cudaGetLastError();

@@ -526,6 +526,7 @@ __device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *
 // store: keep the packed factor in wv.facs for the refinement solves
 template <typename T>
 __global__ void __launch_bounds__(256) k_factor_solve(PlanView pv, WorkView wv, int refine, int store) {
+  grid_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int fail_s;
   const int b = pv.fs_prob[blockIdx.x];
@@ -591,7 +592,7 @@ int launch_factor_solve(const PlanView &pv, const WorkView &wv, const Params &pr
   // which supersedes it (its residual is exact, not that of the assembled S)
   const int refine = (mixed && !store) ? prm.refine_steps : 0;
   cudaFuncSetAttribute(k_factor_solve<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_factor_solve<T><<<pv.B, 256, sm, (cudaStream_t)stream>>>(pv, wv, refine, store);
+  launch(k_factor_solve<T>, pv.B, 256, sm, (cudaStream_t)stream, pv, wv, refine, store);
   ++g_launches;
   return (int)cudaGetLastError();
 }
@@ -601,6 +602,7 @@ int launch_factor_solve(const PlanView &pv, const WorkView &wv, const Params &pr
 template <typename T>
 __global__ void k_backsub(PlanView pv, WorkView wv, Params prm, const double *alpha, double *alpha_out,
                           int gate) {
+  grid_enter();
   const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int slot = threadIdx.x & 31;
   if (c >= pv.n_chunks) return;
@@ -653,7 +655,7 @@ int launch_backsub(const PlanView &pv, const WorkView &wv, const Params &prm, co
                    double *alpha_out, int direct, void *stream) {
   if (pv.n_chunks == 0) return 0;
   const int gate = direct ? GATE_ALL : GATE_RUNNING;
-  k_backsub<T><<<grid_for(pv.n_chunks, 4), 128, 0, (cudaStream_t)stream>>>(pv, wv, prm, alpha, alpha_out, gate);
+  launch(k_backsub<T>, grid_for(pv.n_chunks, 4), 128, 0, (cudaStream_t)stream, pv, wv, prm, alpha, alpha_out, gate);
   ++g_launches;
   return (int)cudaGetLastError();
 }
@@ -666,6 +668,7 @@ int launch_backsub(const PlanView &pv, const WorkView &wv, const Params &prm, co
 template <typename T>
 __global__ void k_update_poses(PlanView pv, WorkView wv, const double *poses, double *out, double scale,
                                int gate, const double *gacc) {
+  grid_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x, p = t >> 2, r = t & 3;
   if (p >= pv.NP) return;
   const int b = pv.pose_prob[p];
@@ -758,7 +761,7 @@ __global__ void k_update_poses(PlanView pv, WorkView wv, const double *poses, do
 template <typename T>
 int launch_update_poses(const PlanView &pv, const WorkView &wv, const double *poses, double *poses_out,
                         double scale, int direct, void *stream, const double *gacc) {
-  k_update_poses<T><<<grid_for(4ll * pv.NP, 128), 128, 0, (cudaStream_t)stream>>>(pv, wv, poses, poses_out, scale,
+  launch(k_update_poses<T>, grid_for(4ll * pv.NP, 128), 128, 0, (cudaStream_t)stream, pv, wv, poses, poses_out, scale,
                                                                        direct ? GATE_ALL : GATE_RUNNING, gacc);
   ++g_launches;
   return (int)cudaGetLastError();
@@ -766,6 +769,7 @@ int launch_update_poses(const PlanView &pv, const WorkView &wv, const double *po
 
 // ---- per-problem LM bookkeeping (thread per problem) ---------------------------
 __global__ void k_reset(PlanView pv, WorkView wv, double lam) {
+  grid_enter();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= pv.B) return;
   LMState s;
@@ -787,7 +791,7 @@ __global__ void k_reset(PlanView pv, WorkView wv, double lam) {
 
 int launch_reset(const PlanView &pv, const WorkView &wv, const Params &prm, double lam, void *stream) {
   (void)prm;
-  k_reset<<<grid_for(pv.B, 128), 128, 0, (cudaStream_t)stream>>>(pv, wv, lam);
+  launch(k_reset, grid_for(pv.B, 128), 128, 0, (cudaStream_t)stream, pv, wv, lam);
   ++g_launches;
   return (int)cudaGetLastError();
 }
@@ -796,6 +800,7 @@ int launch_reset(const PlanView &pv, const WorkView &wv, const Params &prm, doub
 // current (and initial) cost; later linearisation points are accepted candidates
 // whose cost the candidate's cost pass already set
 __global__ void k_post_linearize(PlanView pv, WorkView wv) {
+  grid_enter();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= pv.B) return;
   LMState &s = wv.lm[b];
@@ -810,7 +815,7 @@ __global__ void k_post_linearize(PlanView pv, WorkView wv) {
 }
 
 int launch_post_linearize(const PlanView &pv, const WorkView &wv, void *stream) {
-  k_post_linearize<<<grid_for(pv.B, 128), 128, 0, (cudaStream_t)stream>>>(pv, wv);
+  launch(k_post_linearize, grid_for(pv.B, 128), 128, 0, (cudaStream_t)stream, pv, wv);
   ++g_launches;
   return (int)cudaGetLastError();
 }
@@ -818,6 +823,7 @@ int launch_post_linearize(const PlanView &pv, const WorkView &wv, void *stream) 
 // Nielsen schedule: rho = (F - F') / pred, pred = 0.5 d^T (g + Lambda d).
 // accept (rho > 0): lam *= max(1/3, 1 - (2 rho - 1)^3), nu = 2; else lam *= nu, nu *= 2.
 __global__ void k_decide(PlanView pv, WorkView wv, Params prm) {
+  grid_enter();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= pv.B) return;
   if (wv.lm[b].status != 0) {
@@ -884,13 +890,14 @@ __global__ void k_decide(PlanView pv, WorkView wv, Params prm) {
 }
 
 int launch_decide(const PlanView &pv, const WorkView &wv, const Params &prm, void *stream) {
-  k_decide<<<grid_for(pv.B, 128), 128, 0, (cudaStream_t)stream>>>(pv, wv, prm);
+  launch(k_decide, grid_for(pv.B, 128), 128, 0, (cudaStream_t)stream, pv, wv, prm);
   ++g_launches;
   return (int)cudaGetLastError();
 }
 
 // accepted candidates become the state
 __global__ void k_commit(PlanView pv, WorkView wv, double *poses, double *alpha) {
+  grid_enter();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < pv.NP) {
     const int b = pv.pose_prob[t];
@@ -913,7 +920,7 @@ __global__ void k_commit(PlanView pv, WorkView wv, double *poses, double *alpha)
 
 int launch_commit(const PlanView &pv, const WorkView &wv, double *poses, double *alpha, void *stream) {
   const long long n = pv.NP > pv.L ? pv.NP : pv.L;
-  k_commit<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(pv, wv, poses, alpha);
+  launch(k_commit, grid_for(n, 256), 256, 0, (cudaStream_t)stream, pv, wv, poses, alpha);
   ++g_launches;
   return (int)cudaGetLastError();
 }
@@ -921,6 +928,7 @@ int launch_commit(const PlanView &pv, const WorkView &wv, double *poses, double 
 // dense B (P x L, row-major, problem-local landmark order), C and g_a of one problem
 template <typename T>
 __global__ void k_export_B(PlanView pv, WorkView wv, int b, double *B, double *C, double *ga) {
+  grid_enter();
   const int c = pv.p_chunk_off[b] + blockIdx.x;
   const int N = pv.p_npose[b];
   const int Lb = pv.p_lm_cnt[b], lo = pv.p_lm_off[b];
@@ -944,7 +952,7 @@ template <typename T>
 int launch_export_B_n(const PlanView &pv, const WorkView &wv, int problem, int n_chunks, double *B, double *C,
                       double *ga, void *stream) {
   if (n_chunks == 0) return 0;
-  k_export_B<T><<<n_chunks, 256, 0, (cudaStream_t)stream>>>(pv, wv, problem, B, C, ga);
+  launch(k_export_B<T>, n_chunks, 256, 0, (cudaStream_t)stream, pv, wv, problem, B, C, ga);
   ++g_launches;
   return (int)cudaGetLastError();
 }
@@ -952,6 +960,7 @@ int launch_export_B_n(const PlanView &pv, const WorkView &wv, int problem, int n
 // dense damped reduced system of one problem, FP64 (both triangles), from A, S_L, g, g_L
 template <typename T>
 __global__ void k_export_S(PlanView pv, WorkView wv, int b, double *S, double *gS) {
+  grid_enter();
   const int P = 6 * pv.p_npose[b];
   const size_t off = pv.p_S_off[b];
   const int po = pv.p_param_off[b];
@@ -975,7 +984,7 @@ __global__ void k_export_S(PlanView pv, WorkView wv, int b, double *S, double *g
 template <typename T>
 int launch_export_S(const PlanView &pv, const WorkView &wv, int problem, double *S, double *gS, void *stream) {
   const long long n = (long long)pv.max_P * pv.max_P;
-  k_export_S<T><<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(pv, wv, problem, S, gS);
+  launch(k_export_S<T>, grid_for(n, 256), 256, 0, (cudaStream_t)stream, pv, wv, problem, S, gS);
   ++g_launches;
   // the Schur pass ran for every problem: clear all of S_L / g_L for the next one
   cudaMemsetAsync(wv.SL, 0, (size_t)pv.total_S * sizeof(T), (cudaStream_t)stream);
@@ -986,11 +995,13 @@ template int launch_export_S<float>(const PlanView &, const WorkView &, int, dou
 template int launch_export_S<double>(const PlanView &, const WorkView &, int, double *, double *, void *);
 
 __global__ void k_scale_lambda(PlanView pv, WorkView wv, double factor) {
+  grid_enter();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b < pv.B) wv.lm[b].lam = wv.lm_backup[b].lam * factor;
 }
 
 __global__ void k_take_probe(PlanView pv, WorkView wv, int j) {
+  grid_enter();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= pv.B) return;
   wv.probe_costs[(size_t)j * pv.B + b] = wv.lm[b].status == 0 ? wv.cost_acc[b] : 0.0;
@@ -999,18 +1010,19 @@ __global__ void k_take_probe(PlanView pv, WorkView wv, int j) {
 }
 
 int launch_scale_lambda(const PlanView &pv, const WorkView &wv, double factor, void *stream) {
-  k_scale_lambda<<<grid_for(pv.B, 128), 128, 0, (cudaStream_t)stream>>>(pv, wv, factor);
+  launch(k_scale_lambda, grid_for(pv.B, 128), 128, 0, (cudaStream_t)stream, pv, wv, factor);
   ++g_launches;
   return (int)cudaGetLastError();
 }
 
 int launch_take_probe(const PlanView &pv, const WorkView &wv, int j, void *stream) {
-  k_take_probe<<<grid_for(pv.B, 128), 128, 0, (cudaStream_t)stream>>>(pv, wv, j);
+  launch(k_take_probe, grid_for(pv.B, 128), 128, 0, (cudaStream_t)stream, pv, wv, j);
   ++g_launches;
   return (int)cudaGetLastError();
 }
 
 __global__ void k_to_double(const void *src, int f64, double *dst, int64_t n) {
+  grid_enter();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   dst[i] = f64 ? reinterpret_cast<const double *>(src)[i] : (double)reinterpret_cast<const float *>(src)[i];
@@ -1018,7 +1030,7 @@ __global__ void k_to_double(const void *src, int f64, double *dst, int64_t n) {
 
 int launch_to_double(const void *src, int f64, double *dst, int64_t n, void *stream) {
   if (n <= 0) return 0;
-  k_to_double<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(src, f64, dst, n);
+  launch(k_to_double, grid_for(n, 256), 256, 0, (cudaStream_t)stream, src, f64, dst, n);
   ++g_launches;
   return (int)cudaGetLastError();
 }

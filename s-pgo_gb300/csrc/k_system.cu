@@ -95,6 +95,7 @@ __device__ __forceinline__ void shift_record(V *v, const V *z) {
 // after the other along the chain (101 poses with windows of 41: 202 us with a thread per chain,
 // 12.7 us so).
 __global__ void __launch_bounds__(SPGO_MAX_WINDOW) k_pair_prefix_rec(PlanView pv, WorkView wv) {
+  grid_enter();
   const int b = blockIdx.y;
   if (!problem_active(wv.lm, b, GATE_RELIN)) return;
   __shared__ double v[SPGO_MAX_WINDOW][27];
@@ -143,6 +144,7 @@ __global__ void __launch_bounds__(SPGO_MAX_WINDOW) k_pair_prefix_rec(PlanView pv
 // (all about origin c_i), in place
 template <typename T>
 __global__ void k_pair_suffix(PlanView pv, WorkView wv) {
+  grid_enter();
   const int b = blockIdx.y;
   if (!problem_active(wv.lm, b, GATE_RELIN)) return;
   const int N = pv.p_npose[b], D = pv.p_pair_D[b];
@@ -194,6 +196,7 @@ constexpr int kPrThreads = 896;  // thread per (pose, component) of a 33-pose wi
 constexpr int kShRecs = 32;
 
 __global__ void __launch_bounds__(128) k_pair_shift_df(PlanView pv, WorkView wv) {
+  grid_enter();
   const int b = blockIdx.y;
   if (!problem_active(wv.lm, b, GATE_RELIN)) return;
   __shared__ df v[kShRecs * 27];
@@ -259,6 +262,7 @@ constexpr int kPrWide = 48;
 
 template <int PHASE>
 __global__ void __launch_bounds__(kPrThreads) k_pair_scan_df(PlanView pv, WorkView wv) {
+  grid_enter();
   const int b = blockIdx.x;
   if (!problem_active(wv.lm, b, GATE_RELIN)) return;
   const int N = pv.p_npose[b], D = pv.p_pair_D[b];
@@ -311,6 +315,7 @@ __global__ void __launch_bounds__(kPrThreads) k_pair_scan_df(PlanView pv, WorkVi
 // of F from o to c_i that the mixed path made first (16.6 us a window; 5.2 us so).
 template <typename T>
 __global__ void __launch_bounds__(128) k_pairs_to_A(PlanView pv, WorkView wv) {
+  grid_enter();
   constexpr bool f64 = std::is_same<T, double>::value;
   using V = typename std::conditional<f64, double, df>::type;
   const int b = blockIdx.y;
@@ -414,21 +419,21 @@ int launch_system(const PlanView &pv, const WorkView &wv, int gate, void *stream
   const int nmax = pv.max_P / 6;
   const int nd = pv.max_D > 0 ? pv.max_D : 1;
   if constexpr (std::is_same<T, float>::value) {
-    k_pair_shift_df<<<dim3(grid_for((long long)nmax * nd, kShRecs), pv.B), 4 * kShRecs, 0, st>>>(pv, wv);
+    launch(k_pair_shift_df, dim3(grid_for((long long)nmax * nd, kShRecs), pv.B), 4 * kShRecs, 0, st, pv, wv);
     if (nmax <= kPrWide) {
-      k_pair_scan_df<0><<<pv.B, std::min(kPrThreads, 32 * grid_for(27 * nmax, 32)), 0, st>>>(pv, wv);
+      launch(k_pair_scan_df<0>, pv.B, std::min(kPrThreads, 32 * grid_for(27 * nmax, 32)), 0, st, pv, wv);
     } else {
       const dim3 grid(pv.B, grid_for((long long)nmax * 27, 128));
-      k_pair_scan_df<1><<<grid, 128, 0, st>>>(pv, wv);
-      k_pair_scan_df<2><<<grid, 128, 0, st>>>(pv, wv);
+      launch(k_pair_scan_df<1>, grid, 128, 0, st, pv, wv);
+      launch(k_pair_scan_df<2>, grid, 128, 0, st, pv, wv);
       ++g_launches;
     }
-    k_pairs_to_A<float><<<dim3(grid_for((long long)nmax * nd * 6, 128), pv.B), 128, 0, st>>>(pv, wv);
+    launch(k_pairs_to_A<float>, dim3(grid_for((long long)nmax * nd * 6, 128), pv.B), 128, 0, st, pv, wv);
     g_launches += 3;
   } else {
-    k_pair_prefix_rec<<<dim3(nmax, pv.B), 32 * grid_for(std::min(nd, nmax), 32), 0, st>>>(pv, wv);
-    k_pair_suffix<double><<<dim3(grid_for((long long)nmax * 27, 128), pv.B), 128, 0, st>>>(pv, wv);
-    k_pairs_to_A<double><<<dim3(grid_for((long long)nmax * nd * 6, 128), pv.B), 128, 0, st>>>(pv, wv);
+    launch(k_pair_prefix_rec, dim3(nmax, pv.B), 32 * grid_for(std::min(nd, nmax), 32), 0, st, pv, wv);
+    launch(k_pair_suffix<double>, dim3(grid_for((long long)nmax * 27, 128), pv.B), 128, 0, st, pv, wv);
+    launch(k_pairs_to_A<double>, dim3(grid_for((long long)nmax * nd * 6, 128), pv.B), 128, 0, st, pv, wv);
     g_launches += 3;
   }
   return (int)cudaGetLastError();
@@ -440,6 +445,7 @@ int launch_system(const PlanView &pv, const WorkView &wv, int gate, void *stream
 // partial tiles are added atomically (S_L is cleared by the assembly that reads it).
 template <typename T>
 __global__ void __launch_bounds__(256) k_schur(PlanView pv, WorkView wv, Params prm, int gate) {
+  grid_enter();
   const int w = blockIdx.x;
   const int b = pv.wk_prob[w];
   if (!problem_active(wv.lm, b, gate)) return;
@@ -526,6 +532,7 @@ __global__ void __launch_bounds__(256) k_schur(PlanView pv, WorkView wv, Params 
 // window, whose 6 items left the GPU empty, 235 -> about 90 us.
 // blockIdx.y splits an item's chunks where the plan has too few items to fill the GPU.
 __global__ void __launch_bounds__(256) k_schur_f64(PlanView pv, WorkView wv, Params prm, int gate) {
+  grid_enter();
   const int w = blockIdx.x;
   const int b = pv.wk_prob[w];
   if (!problem_active(wv.lm, b, gate)) return;
@@ -627,9 +634,9 @@ int launch_schur(const PlanView &pv, const WorkView &wv, const Params &prm, void
     // a chunk of one tile keeps an SM's FP64 pipe busy for several microseconds, so items
     // are split down to single chunks until there are four CTAs per SM
     const int sub = std::max(1, std::min(pv.wk_max_len, (4 * kSmCount + pv.n_items - 1) / pv.n_items));
-    k_schur_f64<<<dim3(pv.n_items, sub), 256, 0, (cudaStream_t)stream>>>(pv, wv, prm, GATE_RUNNING);
+    launch(k_schur_f64, dim3(pv.n_items, sub), 256, 0, (cudaStream_t)stream, pv, wv, prm, GATE_RUNNING);
   } else {
-    k_schur<T><<<pv.n_items, 256, 0, (cudaStream_t)stream>>>(pv, wv, prm, GATE_RUNNING);
+    launch(k_schur<T>, pv.n_items, 256, 0, (cudaStream_t)stream, pv, wv, prm, GATE_RUNNING);
   }
   ++g_launches;
   return (int)cudaGetLastError();

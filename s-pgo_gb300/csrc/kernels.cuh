@@ -148,6 +148,33 @@ __device__ __forceinline__ void invert34(const double *T, double *Ti) {
     Ti[4 * i + 3] = -(Ti[4 * i] * T[3] + Ti[4 * i + 1] * T[7] + Ti[4 * i + 2] * T[11]);
 }
 
+// Every kernel of the solver opens with this.  Its grid may have been launched while the one before
+// it in the stream still ran (launch() below): wait until that one has finished and its writes are
+// visible (it waited for its own predecessor first, so everything earlier has too), then let the
+// next grid's CTAs come in as soon as all of this one's have started.
+__device__ __forceinline__ void grid_enter() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// k<<<grid, block, smem, st>>>(args) with programmatic stream serialization: the launch overlaps
+// the end of the grid before it.  An LM iteration is some twenty small dependent kernels
+// (GN step of a 10-pose window: 121 us launched plainly, 104 us so).
+template <typename... P, typename... A>
+inline void launch(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);  // (an error is read by cudaGetLastError)
+}
+
 inline int grid_for(long long n, int block) { return (int)((n + block - 1) / block); }
 
 }  // namespace spgo
