@@ -432,14 +432,18 @@ int launch_chain(const PlanView &pv, const WorkView &wv, const double *poses, in
   return (int)cudaGetLastError();
 }
 
-constexpr int kCostThreads = 64;   // short CTAs, many per SM (latency-bound)
+// Latency-bound: short CTAs, many per SM, where there are enough chunks to fill it (64 windows of
+// 3731 chunks: 10.76 ms with 64 threads, 10.93 with 128, 11.33 with 256); twice the threads while
+// all CTAs are resident at once, eight to an SM, and the longest chunk is what takes the time
+// (GN step of 22 chunks: 104 us with 64, 92 with 128 or 256; LM step of 672: 1276, 1235, 1236).
+constexpr int kCostThreads = 64, kCostThreadsFew = 128, kCostFew = 8 * 152;
 
 template <typename T>
 int launch_linearize(const PlanView &pv, const WorkView &wv, const Params &prm, const double *alpha,
                      int cost_only, int gate, void *stream) {
   if (pv.n_chunks == 0) return 0;
   if (!cost_only) return launch_jacobian<T>(pv, wv, prm, alpha, gate, stream);
-  const int nt = prm.cost_block > 0 ? prm.cost_block : kCostThreads;
+  const int nt = prm.cost_block > 0 ? prm.cost_block : pv.n_chunks <= kCostFew ? kCostThreadsFew : kCostThreads;
   size_t dc;
   launch(k_cost<T>, pv.n_chunks, nt, cost_smem<T>(pv.max_nb, &dc), (cudaStream_t)stream, pv, wv, prm, alpha, gate);
   ++g_launches;
