@@ -45,16 +45,6 @@
 
 namespace spgo {
 
-// left camera of frame f: rotation (cam -> world) and centre, FP64 from the
-// double-float frame tables of the mixed path
-__device__ __forceinline__ void frame_Rc(const WorkView &wv, int f, double *R, double *c) {
-  const float *Rh = wv.fr_Rf + (size_t)f * 18, *Rl = wv.fr_Rl + (size_t)f * 18;
-#pragma unroll
-  for (int k = 0; k < 9; ++k) R[k] = (double)Rh[k] + (double)Rl[k];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) c[k] = wv.fr_c[(size_t)f * 6 + k];
-}
-
 // a problem takes (the next step of) the refinement: running, its step not failed, and
 // its refinement not yet converged (outer_tol)
 __device__ __forceinline__ bool refine_active(const WorkView &wv, int b) {
@@ -652,12 +642,13 @@ __global__ void __launch_bounds__(kRsThreads) k_resid_solve(PlanView pv, WorkVie
 // ---- the same reduction for wide problems, spread over the GPU ----------------------
 // One CTA per problem puts a wide problem's FP64 pair sums on one SM (GB300 issues FP64
 // at 1/64 of its FP32 rate): for P = 3000 that was 267 us per refinement step.  Here
-//   k_rs_sums_large   thread per (pose, component): the row sums (over hi) and the
+//   k_rs_sums_large   four lanes per (pose, component): the row sums (over hi) and the
 //                     column sums (over lo, moved to c_lo) of the pair duals, into lg_red
 //   k_rs_scan_large   one CTA: the rows' prefix over the poses, as segment sums, an
 //                     exclusive scan of the segments and a second walk of each segment
-//   k_rs_rhs_large    thread per pose: the world-to-pose transform, the right-hand side
+//   k_rs_rhs_large    thread per unknown: the world-to-pose transform, the right-hand side
 //                     into lg_y for the multi-CTA substitutions; clears the pair duals
+// (100 poses with windows of 41: 20.1 and 8.3 us with a thread per sum and per pose, 7.8 and 5.1 us so)
 // The per-pose values are those of k_resid_solve; only the prefix is summed in another
 // order (FP64, segments of ~N / 42 poses).
 // (FP64-bound: small CTAs spread the sums over the SMs, and the centres come as FP64)
@@ -665,37 +656,47 @@ __global__ void __launch_bounds__(64) k_rs_sums_large(PlanView pv, WorkView wv, 
   grid_enter();
   if (!refine_active(wv, b)) return;
   const int N = pv.p_npose[b], D = pv.p_pair_D[b], fo = pv.p_frame_off[b];
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 12 * N) return;
+  // row sums of all components, then columns' m_v, then columns' m_w, each kind from a warp's
+  // first lane on
+  const int wr = (6 * N + 7) / 8, wc = (3 * N + 7) / 8, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int kind = w < wr ? 0 : w < wr + wc ? 1 : 2, part = threadIdx.x & 3;
+  const int g = 8 * (w - (kind == 0 ? 0 : kind == 1 ? wr : wr + wc)) + ((threadIdx.x & 31) >> 2);
   double *rowm = wv.lg_red + ((size_t)pv.p_pose_off[b] + b) * 12, *colm = rowm + (size_t)(N + 1) * 6;
   const double *recs = wv.pdual + (size_t)pv.p_pair_off[b] * 6;
   auto cen = [&](int f, int k) { return wv.fr_c[(size_t)(fo + f) * 6 + k]; };
-  const int k = t % 6;
-  if (t < 6 * N) {  // row lo = t / 6
-    const int lo = t / 6;
-    const double *r = recs + (size_t)lo * D * 6 + k;
-    const int nd = min(D, N - lo);
-    double acc = 0.0;
+  double acc = 0.0;
+  double *out = nullptr;
+  if (kind == 0) {
+    const int lo = g / 6, k = g % 6;
+    if (lo < N) {
+      const double *r = recs + (size_t)lo * D * 6 + k;
+      const int nd = min(D, N - lo);
 #pragma unroll 4
-    for (int d = 0; d < nd; ++d) acc += r[(size_t)d * 6];
-    rowm[lo * 6 + k] = acc;
-    if (lo == 0) colm[k] = 0.0;  // no record ends at pose 0
-  } else {  // column hi = (t - 6 N) / 6 + 1
-    const int hi = (t - 6 * N) / 6 + 1;
-    double acc = 0.0;
-    if (k < 3) {
-      const int k1 = (k + 1) % 3, k2 = (k + 2) % 3;
-#pragma unroll 4
-      for (int lo = max(0, hi - D); lo < hi; ++lo) {
-        const double *r = recs + ((size_t)lo * D + (hi - lo - 1)) * 6;
-        acc += r[k] + (cen(lo, k1) * r[3 + k2] - cen(lo, k2) * r[3 + k1]);
-      }
-    } else {
-#pragma unroll 4
-      for (int lo = max(0, hi - D); lo < hi; ++lo) acc += recs[((size_t)lo * D + (hi - lo - 1)) * 6 + k];
+      for (int d = part; d < nd; d += 4) acc += r[(size_t)d * 6];
+      out = rowm + lo * 6 + k;
+      if (lo == 0 && part == 0) colm[k] = 0.0;  // no record ends at pose 0
     }
-    colm[hi * 6 + k] = acc;
+  } else {
+    const int hi = g / 3 + 1, k = g % 3;
+    if (hi <= N) {
+      if (kind == 1) {
+#pragma unroll 4
+        for (int lo = max(0, hi - D) + part; lo < hi; lo += 4) acc += recs[((size_t)lo * D + (hi - lo - 1)) * 6 + 3 + k];
+        out = colm + hi * 6 + 3 + k;
+      } else {
+        const int k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1;
+#pragma unroll 4
+        for (int lo = max(0, hi - D) + part; lo < hi; lo += 4) {
+          const double *r = recs + ((size_t)lo * D + (hi - lo - 1)) * 6;
+          acc = fma(-cen(lo, k2), r[3 + k1], fma(cen(lo, k1), r[3 + k2], acc + r[k]));
+        }
+        out = colm + hi * 6 + k;
+      }
+    }
   }
+  acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+  acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+  if (out && part == 0) *out = acc;
 }
 
 constexpr int kScanSegs = 42;  // segments per component: 6 x 42 = 252 of the 256 threads
@@ -759,39 +760,37 @@ __global__ void __launch_bounds__(64) k_rs_rhs_large(PlanView pv, WorkView wv, i
   // the pair duals are summed: cleared for the next pass
   double *recs = wv.pdual + (size_t)pv.p_pair_off[b] * 6;
   for (size_t q = t; q < (size_t)N * D * 6; q += (size_t)gridDim.x * blockDim.x) recs[q] = 0.0;
-  if (t >= N) return;
-  const int i = t;
-  const double lam = wv.lm[b].lam;
+  if (t >= P) return;
+  const int i = t / 6, k = t % 6, r = k < 3 ? k : k - 3;
   const float *A = reinterpret_cast<const float *>(wv.A) + pv.p_S_off[b];
-  double R[9], ci[3];
-  frame_Rc(wv, fo + i, R, ci);
-  const double *S = rowm + i * 6;
-  const double w[3] = {S[0] - (ci[1] * S[5] - ci[2] * S[4]), S[1] - (ci[2] * S[3] - ci[0] * S[5]),
-                       S[2] - (ci[0] * S[4] - ci[1] * S[3])};
-  double out[6];
+  const float *Rh = wv.fr_Rf + (size_t)(fo + i) * 18 + r, *Rl = wv.fr_Rl + (size_t)(fo + i) * 18 + r;
+  const double *c = wv.fr_c + (size_t)(fo + i) * 6, *S = rowm + i * 6;
+  double m[3];  // m_w about c_i, or m_v
+  if (k < 3) {
+    m[0] = S[0] - (c[1] * S[5] - c[2] * S[4]);
+    m[1] = S[1] - (c[2] * S[3] - c[0] * S[5]);
+    m[2] = S[2] - (c[0] * S[4] - c[1] * S[3]);
+  } else {
 #pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    out[r] = R[r] * w[0] + R[3 + r] * w[1] + R[6 + r] * w[2];
-    out[3 + r] = R[r] * S[3] + R[3 + r] * S[4] + R[6 + r] * S[5];
+    for (int q = 0; q < 3; ++q) m[q] = S[3 + q];
   }
+  double out = 0.0;
 #pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    const int p = 6 * i + k;
-    const double x = wv.delta[po + p];
-    const double rhs = out[k] - lam * (double)A[(size_t)p * P + p] * x - (double)wv.rhsB[po + p];
-    wv.rhsB[po + p] = 0.f;
-    reinterpret_cast<float *>(wv.lg_y)[po + p] = (float)rhs;
-  }
+  for (int q = 0; q < 3; ++q) out += ((double)Rh[3 * q] + (double)Rl[3 * q]) * m[q];
+  const double x = wv.delta[po + t];
+  const double rhs = out - wv.lm[b].lam * (double)A[(size_t)t * P + t] * x - (double)wv.rhsB[po + t];
+  wv.rhsB[po + t] = 0.f;
+  reinterpret_cast<float *>(wv.lg_y)[po + t] = (float)rhs;
 }
 
 int launch_resid_reduce_large(const PlanView &pv, const WorkView &wv, int b, int N, void *stream) {
   if (!wv.lg_red) return 0;  // (the FP64 path has no refinement)
   cudaStream_t st = (cudaStream_t)stream;
-  launch(k_rs_sums_large, (12 * N + 63) / 64, 64, 0, st, pv, wv, b);
+  launch(k_rs_sums_large, ((6 * N + 7) / 8 + 2 * ((3 * N + 7) / 8) + 1) / 2, 64, 0, st, pv, wv, b);  // (a warp per 8 sums)
   const size_t sm = (size_t)N * 6 * sizeof(double);
   cudaFuncSetAttribute(k_rs_scan_large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   launch(k_rs_scan_large, 1, 256, sm, st, pv, wv, b);
-  launch(k_rs_rhs_large, std::max((N + 63) / 64, 96), 64, 0, st, pv, wv, b);  // (the clearing wants the CTAs)
+  launch(k_rs_rhs_large, std::max((6 * N + 63) / 64, 96), 64, 0, st, pv, wv, b);  // (the clearing wants the CTAs)
   g_launches += 3;
   return (int)cudaGetLastError();
 }
