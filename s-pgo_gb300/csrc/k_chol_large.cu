@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kLgNB) k_lg_potrf_rows(PlanView pv, WorkView w
     __syncthreads();
     const float d = c[k];
     bad = bad || !(d > 0.f) || !(d < INFINITY);
-    const float lkk = sqrtf(d), rinv = 1.f / lkk;  // correctly rounded, as in the batched factorisation
+    const float lkk = sqrtf(d), rinv = 1.f / lkk;  // correctly rounded
     if (i == k) {
       a[k] = lkk;
       rdiag = rinv;

@@ -1030,7 +1030,7 @@ __global__ void k_to_double(const void *src, int f64, double *dst, int64_t n) {
 
 int launch_to_double(const void *src, int f64, double *dst, int64_t n, void *stream) {
   if (n <= 0) return 0;
-  launch(k_to_double, grid_for(n, 256), 256, 0, (cudaStream_t)stream, src, f64, dst, n);
+  k_to_double<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(src, f64, dst, n);
   ++g_launches;
   return (int)cudaGetLastError();
 }

@@ -157,14 +157,19 @@ __device__ __forceinline__ void grid_enter() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// k<<<grid, block, smem, st>>>(args) with programmatic stream serialization: the launch overlaps
-// the end of the grid before it.  An LM iteration is some twenty small dependent kernels
-// (GN step of a 10-pose window: 121 us launched plainly, 104 us so).
+// k<<<grid, block, smem, st>>>(pv, args) with programmatic stream serialization: the launch
+// overlaps the end of the grid before it.  An LM iteration is some twenty small dependent kernels
+// (GN step of a 10-pose window: 121 us launched plainly, 104 us so; 100 trials of
+// 465 thousand observations: 264 and 244).  Plain beyond kOverlapObs observations, where the gaps are nothing
+// and the early CTAs take room from the second stream's (64 windows of 1.4 million observations:
+// 10.73 ms plain, 10.82 overlapped; 256 of 3.7 million, two iterations: 3139 and 3242 us).
+constexpr int64_t kOverlapObs = 1000000;
+
 template <typename... P, typename... A>
-inline void launch(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+inline void launch(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const PlanView &pv, A... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+  attr.val.programmaticStreamSerializationAllowed = pv.O <= kOverlapObs;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -172,7 +177,8 @@ inline void launch(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStre
   cfg.stream = st;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  (void)cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);  // (an error is read by cudaGetLastError)
+  // (an error is read by cudaGetLastError)
+  (void)cudaLaunchKernelEx(&cfg, k, pv, static_cast<A>(args)...);
 }
 
 inline int grid_for(long long n, int block) { return (int)((n + block - 1) / block); }
