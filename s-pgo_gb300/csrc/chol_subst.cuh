@@ -8,10 +8,9 @@
 // more than it saves, and with dinv[k] = 1 / L(k, k) besides).
 #pragma once
 #include "kernels.cuh"
+#include "subst_index.h"
 
 namespace spgo {
-
-constexpr int kPanel = 16;  // block width of the factorisation and the substitutions
 
 // 1 / d and 1 / sqrt(d) for an FP64 pivot.  The pivots are the serial chain of a factorisation,
 // and one FP64 instruction of a warp, a comparison or a conversion too, holds its quarter of an
@@ -67,10 +66,9 @@ __device__ void chol_substitute(const T *Lm, const int *cb, T *y, const T *dinv,
   const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31;
   const int i = lane & 15, h = (lane >> 4) * kHalf;  // lanes (i, h): unknown i, terms h .. h + 7
   const unsigned all = 0xffffffffu;
-  // offset of column c of a block from its first one's: cb[kb + c] - cb[kb]
-  auto col = [&](int kb, int c) { return c * (P - kb) - c * (c + 1) / 2; };
-  // (loads are unconditional, their values selected: a predicated load costs a branch.  Rows and
-  // columns past a narrow last block reach up to kPanel elements behind the factor and y.)
+  // (loads are unconditional, their values selected: a predicated load costs a branch.  Rows past a
+  // narrow last block reach up to kPanel elements behind the factor and y; columns past it are
+  // its last column's, subst_index.h.)
   T d[kD], s[kHalf], v = T(0);  // warp 0: the block to solve, the block between it and the next, its right-hand side
   // sum over the 16 lanes' u of the coefficients c
   auto product = [&](const T (&c)[kHalf], T u) {
@@ -82,12 +80,12 @@ __device__ void chol_substitute(const T *Lm, const int *cb, T *y, const T *dinv,
   // forward L z = y
   auto load_fwd = [&](int kb, int w) {
     const int c0 = kUnit ? 0 : h;
-    const T *B = Lm + ix(kb + i, kb) + col(kb, c0);
+    const T *B = Lm + ix(kb + i, kb) + subst_fwd_first(P, kb, c0);
 #pragma unroll
     for (int q = 0; q < kD; ++q) {
       const T x = *B;
       d[q] = i < w && c0 + q < i + (kUnit ? 0 : 1) ? x : T(0);
-      B += P - kb - 1 - c0 - q;
+      B += subst_fwd_step(P, kb, c0 + q);
     }
   };
   if (warp == 0) {
@@ -107,7 +105,7 @@ __device__ void chol_substitute(const T *Lm, const int *cb, T *y, const T *dinv,
       if (lane < w) y[kb + lane] = v;
       if (ke < P) {
         load_fwd(ke, min(kPanel, P - ke));
-        const T *B = Lm + ix(ke + i, kb) + col(kb, h);
+        const T *B = Lm + ix(ke + i, kb) + subst_col(P, kb, h);
 #pragma unroll
         for (int q = 0; q < kHalf; ++q) {
           const T x = *B;
