@@ -348,10 +348,11 @@ __global__ void __launch_bounds__(256) k_lg_fwd(PlanView pv, WorkView wv, int b,
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   __shared__ T part[4][kLgNB];
   __shared__ T zs[kLgNB];
-  // the diagonal block (strictly lower, its two 32-wide diagonal parts of the unit factor, so that
-  // the chain is one shuffle and one FMA per unknown) and the pivots' reciprocals,
+  // staged while the earlier blocks are still being solved: the diagonal block (strictly lower, its
+  // two 32-wide diagonal parts of the unit factor, so that the chain is one shuffle and one FMA per
+  // unknown) and the pivots' reciprocals
   __shared__ T Ld[kLgNB][kLgNB + 1];
-  __shared__ T ds[kLgNB];             // staged while the earlier blocks are still being solved
+  __shared__ T ds[kLgNB];
   __shared__ int timed_out;
   const int P = 6 * pv.p_npose[b], po = pv.p_param_off[b];
   const int k = blockIdx.x, kb = k * kLgNB, nb = min(kLgNB, P - kb);
@@ -441,10 +442,11 @@ __global__ void __launch_bounds__(256) k_lg_bwd(PlanView pv, WorkView wv, int b,
   if (!problem_active(wv.lm, b, GATE_RUNNING)) return;
   __shared__ T part[4][kLgNB];
   __shared__ T zs[kLgNB];
-  // the diagonal block (strictly lower, its two 32-wide diagonal parts of the unit factor, so that
-  // the chain is one shuffle and one FMA per unknown) and the pivots' reciprocals,
+  // staged while the later blocks are still being solved: the diagonal block (strictly lower, its
+  // two 32-wide diagonal parts of the unit factor, so that the chain is one shuffle and one FMA per
+  // unknown) and the pivots' reciprocals
   __shared__ T Ld[kLgNB][kLgNB + 1];
-  __shared__ T ds[kLgNB];             // staged while the later blocks are still being solved
+  __shared__ T ds[kLgNB];
   __shared__ int timed_out;
   const int P = 6 * pv.p_npose[b], po = pv.p_param_off[b];
   const int nblk = (P + kLgNB - 1) / kLgNB, k = nblk - 1 - (int)blockIdx.x;

@@ -423,11 +423,12 @@ __global__ void __launch_bounds__(3 * kChainDfFrames) k_chain_df(PlanView pv, Wo
 }
 
 int launch_chain(const PlanView &pv, const WorkView &wv, const double *poses, int gate, int f64, void *stream) {
+  cudaStream_t st = (cudaStream_t)stream;
+  const int warps = std::max(1, (pv.max_P / 6 + 31) / 32);  // of frames, three threads each
   if (f64)
-    launch(k_chain, pv.B, 96 * std::min(kChainFrames / 32, std::max(1, (pv.max_P / 6 + 31) / 32)), 0, (cudaStream_t)stream, 
-        pv, wv, poses, gate);
+    launch(k_chain, pv.B, 96 * std::min(kChainFrames / 32, warps), 0, st, pv, wv, poses, gate);
   else
-    launch(k_chain_df, pv.B, 96 * std::min(kChainDfFrames / 32, std::max(1, (pv.max_P / 6 + 31) / 32)), 0, (cudaStream_t)stream, pv, wv, poses, gate);
+    launch(k_chain_df, pv.B, 96 * std::min(kChainDfFrames / 32, warps), 0, st, pv, wv, poses, gate);
   ++g_launches;
   return (int)cudaGetLastError();
 }
@@ -436,7 +437,7 @@ int launch_chain(const PlanView &pv, const WorkView &wv, const double *poses, in
 // 3731 chunks: 10.76 ms with 64 threads, 10.93 with 128, 11.33 with 256); twice the threads while
 // all CTAs are resident at once, eight to an SM, and the longest chunk is what takes the time
 // (GN step of 22 chunks: 104 us with 64, 92 with 128 or 256; LM step of 672: 1276, 1235, 1236).
-constexpr int kCostThreads = 64, kCostThreadsFew = 128, kCostFew = 8 * 152;
+constexpr int kCostThreads = 64, kCostThreadsFew = 128, kCostFew = 8 * kSmCount;
 
 template <typename T>
 int launch_linearize(const PlanView &pv, const WorkView &wv, const Params &prm, const double *alpha,

@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kTwThreads) k_pair_twists(PlanView pv, WorkVie
 int launch_pair_twists(const PlanView &pv, const WorkView &wv, void *stream) {
   const int nmax = pv.max_P / 6;
   int slice = kTwSlice;
-  while (slice > 8 && (long long)pv.B * ((nmax + slice - 1) / slice) < 152) slice /= 2;
+  while (slice > 8 && (long long)pv.B * ((nmax + slice - 1) / slice) < kSmCount) slice /= 2;
   launch(k_pair_twists, dim3(pv.B, (nmax + slice - 1) / slice), kTwThreads, 0, (cudaStream_t)stream, pv, wv, slice);
   ++g_launches;
   return (int)cudaGetLastError();

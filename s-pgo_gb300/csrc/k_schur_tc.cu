@@ -344,7 +344,7 @@ size_t tc_smem_bytes() { return sizeof(TcSmem) + 1024; }
 // 20-pose window, a chunk per CTA: 66 -> 14 us; 100 items of 35 chunks: two shares each took
 // 52 us, whole ones 44).
 static int tc_shares(const PlanView &pv) {
-  constexpr float kFixed = 13.f, kSms = 152.f;
+  constexpr float kFixed = 13.f, kSms = (float)kSmCount;
   const float n = (float)pv.n_tc_items, mean = (float)pv.n_tc_chunks / n;
   int best = 1;
   float t_best = 1e30f;

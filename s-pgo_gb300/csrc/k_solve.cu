@@ -263,53 +263,53 @@ __device__ void factor_solve_body(T *Lm, const int *cb, T *y, double *x, float *
   const int ld = (P + 3) & ~3;
   auto update_tiles = [&](int ke, int wi, int nwu) {
     if constexpr (!kF64) {
-    const int R = P - ke, lr = lane & 7, lc = lane >> 3;
-    int turn = wi;
-    for (int j0 = 0; j0 < R; j0 += 16)
-      for (int i0 = j0 & ~31; i0 < R; i0 += 32) {
-        if (turn-- != 0) continue;
-        turn = nwu - 1;
-        // (rows and columns past the end take the last one's place and are dropped)
-        const float *cols = stage + min(j0 + 4 * lc, ld - 4);
-        const float *rows[4];
+      const int R = P - ke, lr = lane & 7, lc = lane >> 3;
+      int turn = wi;
+      for (int j0 = 0; j0 < R; j0 += 16)
+        for (int i0 = j0 & ~31; i0 < R; i0 += 32) {
+          if (turn-- != 0) continue;
+          turn = nwu - 1;
+          // (rows and columns past the end take the last one's place and are dropped)
+          const float *cols = stage + min(j0 + 4 * lc, ld - 4);
+          const float *rows[4];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) rows[a] = stage + min(i0 + lr + 8 * a, R - 1);
-        float acc[4][4] = {};
+          for (int a = 0; a < 4; ++a) rows[a] = stage + min(i0 + lr + 8 * a, R - 1);
+          float acc[4][4] = {};
 #pragma unroll
-        for (int k0 = 0; k0 < kPanel; k0 += 4) {  // (loads of four columns first)
-          float4 c[4];
-          float x[4][4];
+          for (int k0 = 0; k0 < kPanel; k0 += 4) {  // (loads of four columns first)
+            float4 c[4];
+            float x[4][4];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            c[q] = *reinterpret_cast<const float4 *>(cols + (k0 + q) * ld);
+            for (int q = 0; q < 4; ++q) {
+              c[q] = *reinterpret_cast<const float4 *>(cols + (k0 + q) * ld);
 #pragma unroll
-            for (int a = 0; a < 4; ++a) x[q][a] = rows[a][(k0 + q) * ld];
+              for (int a = 0; a < 4; ++a) x[q][a] = rows[a][(k0 + q) * ld];
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+              for (int a = 0; a < 4; ++a) {
+                acc[a][0] = fmaf(x[q][a], c[q].x, acc[a][0]);
+                acc[a][1] = fmaf(x[q][a], c[q].y, acc[a][1]);
+                acc[a][2] = fmaf(x[q][a], c[q].z, acc[a][2]);
+                acc[a][3] = fmaf(x[q][a], c[q].w, acc[a][3]);
+              }
+          }
+          float *dst[4], old[4][4];
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            dst[b] = Lm + ix(ke + i0 + lr, ke + min(j0 + 4 * lc + b, R - 1));
+#pragma unroll
+            for (int a = 0; a < 4; ++a) old[a][b] = dst[b][min(8 * a, R - 1 - i0 - lr)];
           }
 #pragma unroll
-          for (int q = 0; q < 4; ++q)
+          for (int b = 0; b < 4; ++b)
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-              acc[a][0] = fmaf(x[q][a], c[q].x, acc[a][0]);
-              acc[a][1] = fmaf(x[q][a], c[q].y, acc[a][1]);
-              acc[a][2] = fmaf(x[q][a], c[q].z, acc[a][2]);
-              acc[a][3] = fmaf(x[q][a], c[q].w, acc[a][3]);
+              const int i = i0 + lr + 8 * a;
+              if (i >= j0 + 4 * lc + b && i >= kPanel && i < R) dst[b][8 * a] = old[a][b] - acc[a][b];
             }
         }
-        float *dst[4], old[4][4];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          dst[b] = Lm + ix(ke + i0 + lr, ke + min(j0 + 4 * lc + b, R - 1));
-#pragma unroll
-          for (int a = 0; a < 4; ++a) old[a][b] = dst[b][min(8 * a, R - 1 - i0 - lr)];
-        }
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-#pragma unroll
-          for (int a = 0; a < 4; ++a) {
-            const int i = i0 + lr + 8 * a;
-            if (i >= j0 + 4 * lc + b && i >= kPanel && i < R) dst[b][8 * a] = old[a][b] - acc[a][b];
-          }
-      }
     }
   };
   // right-looking with one block of look-ahead: once block kb's rows are solved, the next

@@ -625,8 +625,6 @@ __global__ void __launch_bounds__(256) k_schur_f64(PlanView pv, WorkView wv, Par
   }
 }
 
-constexpr int kSmCount = 152;
-
 template <typename T>
 int launch_schur(const PlanView &pv, const WorkView &wv, const Params &prm, void *stream) {
   if (pv.n_items == 0) return 0;

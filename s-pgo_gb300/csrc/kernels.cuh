@@ -181,6 +181,8 @@ inline void launch(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStre
   (void)cudaLaunchKernelEx(&cfg, k, pv, static_cast<A>(args)...);
 }
 
+constexpr int kSmCount = 152;  // SMs of a GB300 (two dies of 76)
+
 inline int grid_for(long long n, int block) { return (int)((n + block - 1) / block); }
 
 }  // namespace spgo

@@ -166,8 +166,9 @@ class Controller:
                                        _vp(out), _vp(cache), st), "mlp_grad")
 
     def train(self, tr: Traces, epochs=60, batch=512, lr=2e-3, seed=0, fit_norm=True) -> List[float]:
-        """Adam on the mean loss; the standardised traces stay on the device and
-        every step is three kernel launches (forward, backward, Adam)."""
+        """Adam on the mean loss; the standardised traces stay on the device and every step is
+        three of the library's kernels (forward, loss and gradient; their sum over the CTAs;
+        Adam)."""
         if fit_norm:
             self.fit_normalization(tr.X)
         n = tr.X.shape[0]
