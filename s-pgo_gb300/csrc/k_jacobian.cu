@@ -19,7 +19,7 @@
 // thousands of observations put errors into A and W that, measured against S, reach its
 // smallest eigenvalues (an FP32-assembled S of a badly initialised circle problem came out
 // indefinite where the FP64 one has scaled smallest eigenvalue 4e-4).  So there H and h are
-// exact sums (two-product, double-float) of rows rounded once to FP32, every further value is
+// exact sums (two-product, double-float) over FP32 rows, every further value is
 // a double-float, a warp's run over the observations of one target frame is summed in
 // double-float and goes to the FP64 pair record by an FP64 atomic (the pair reduction then
 // runs in double-float about one origin, k_system.cu), and the slab is rounded to FP32 once,

@@ -257,7 +257,8 @@ __global__ void __launch_bounds__(128) k_pair_shift_df(PlanView pv, WorkView wv)
 // 2. thread per (i, component): suffix over hi, F(i, i + e) = sum_{d > e} P(i, i + d).
 // PHASE 0: both, one CTA per problem (the windows of a batch); 1, 2: one of them over a grid,
 // for trajectories of more than kPrWide poses (500 poses on one SM took 150 us, spread out
-// 12 us; at 32 poses one CTA's barrier is cheaper than a second launch).
+// 12 us).  Whole Gauss-Newton steps with one launch and with two, us: a 10-pose window 86 and 88,
+// 64 of 10 105 and 108, 64 of 32 392 and 396; 48 poses 277 and 272, 100 poses 321 and 297.
 constexpr int kPrWide = 48;
 
 template <int PHASE>

@@ -159,10 +159,14 @@ __device__ __forceinline__ void grid_enter() {
 
 // k<<<grid, block, smem, st>>>(pv, args) with programmatic stream serialization: the launch
 // overlaps the end of the grid before it.  An LM iteration is some twenty small dependent kernels
-// (GN step of a 10-pose window: 121 us launched plainly, 104 us so; 100 trials of
-// 465 thousand observations: 264 and 244).  Plain beyond kOverlapObs observations, where the gaps are nothing
-// and the early CTAs take room from the second stream's (64 windows of 1.4 million observations:
-// 10.73 ms plain, 10.82 overlapped; 256 of 3.7 million, two iterations: 3139 and 3242 us).
+// (GN step of a 10-pose window: 121 us launched plainly, 104 us so; 100 trials of 465 thousand
+// observations: 264 and 244).  Plain beyond kOverlapObs observations, where a batch's gaps are
+// nothing and the early CTAs take room from the second stream's (64 windows of 0.8 million
+// observations, two LM iterations: 1052 us plain, 1058 overlapped; 128 of 1.7 million: 1732 and
+// 1794; 256 of 3.7 million: 3139 and 3242).  Observations stand in for the number of problems: one
+// or a few wide problems beyond the line would still gain (two LM iterations, plain and overlapped:
+// 60 poses with windows of 44, 1.2 million, 1292 and 1256 us; four of 100 poses, 1.5 million, 2665
+// and 2617; 500 poses, 3.9 million, 3594 and 3583).
 constexpr int64_t kOverlapObs = 1000000;
 
 template <typename... P, typename... A>
