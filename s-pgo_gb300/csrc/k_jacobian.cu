@@ -26,9 +26,10 @@
 // at the end.  The refinement's residual pass (k_refine.cu) uses the same rounded rows in the
 // same structure: where S's small eigenvalues are at the FP32 rounding of A, a preconditioner
 // from another rounding of the same Jacobian is no preconditioner (three problems of the
-// 256-window batch stalled up to 2.8x above the FP64 cost).  (A slab accumulated in FP32, and one whose double-float moments were rounded
-// before an FP32 rotation to the pose axes, left single ill-conditioned problems of the
-// 256-window batch with an unusable preconditioner.)  The residuals, camera-frame points and
+// 256-window batch stalled up to 2.8x above the FP64 cost).  (A slab accumulated in FP32, and
+// one whose double-float moments were rounded before an FP32 rotation to the pose axes, left
+// single ill-conditioned problems of the 256-window batch with an unusable preconditioner.)
+// The residuals, camera-frame points and
 // anchor points are the cost pass's at the same state, rounded once from double-float.  The
 // FP64 path is the same kernel in double, forming those itself.
 //

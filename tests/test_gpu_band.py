@@ -1,8 +1,8 @@
 """The banded factorisation of wide reduced systems (mixed path): windows of D poses give a
-band of 6 D - 1, eliminated from both ends in 16-wide blocks.  Sizes at the edges of its
-route: one block of band, a band that is and is not a multiple of 16, padding of every
-residue (P mod 16), systems barely wider than the band (one elimination only), the widest
-band it takes and one above it (the multi-CTA path).  The refined mixed step must match the
+band of 6 D - 1, eliminated from both ends in 16-wide blocks.  Bands of one block to the 17 it
+takes and one wider (the multi-CTA path), seven of the eight residues P mod 16, systems barely
+wider than the band (``test_gpu_band_edges.py``: the eighth, the smallest system and both sides
+of the route's line).  The refined mixed step must match the
 FP64 path's step from the same state.  Tolerance: the mixed step's stated accuracy, 1e-5 of
 the step (its refinement's floor is the FP32 rounding of the Jacobian, 1e-7 to 2e-6)."""
 import numpy as np

@@ -1,12 +1,13 @@
 """Failure paths that must end in a status, not a hang or a NaN.
 
-The bounded device-side waits (the multi-CTA substitutions of wide reduced systems,
-the tensor-core Schur pipeline) give up after ``spgo_params.wait_us``.  Shortening
-that limit to one microsecond makes the substitutions' waits for earlier blocks run
-out: the step must be rejected, counted as a timeout (not as a factorisation
-failure), and leave the state finite; with the default limit restored the same
-solver must solve normally.  Nothing here faults, traps or hangs the GPU: every wait
-stays bounded, only its limit changes.
+The bounded device-side waits (the solves of wide reduced systems, the tensor-core
+Schur pipeline) give up after ``spgo_params.wait_us``.  Shortening that limit to one
+microsecond makes the waits of a wide mixed problem run out (today the banded path's
+and the Schur pipeline's; ``test_gpu_wait_limits.py`` takes each kind by itself): the
+step must be rejected, counted as a timeout (not as a factorisation failure), and
+leave the state finite; with the default limit restored the same solver must solve
+normally.  Nothing here faults, traps or hangs the GPU: every wait stays bounded, only
+its limit changes.
 """
 import numpy as np
 import pytest
