@@ -49,8 +49,7 @@ constexpr int kBandStages = 5;
 static_assert((SPGO_BAND_MAX_H + 2) * (SPGO_BAND_MAX_H + 3) / 2 * kBandSlot * 4 <= 220 * 1024, "shared memory");
 static_assert((SPGO_BAND_MAX_H + 1) * kBb + 32 <= kBandSolveThreads, "blocks 2..h below the diagonal, and the next");
 
-// the two ends' block counts: [0, mL) from the first, [mR, nB) from the second, each at least one
-// (band_route)
+// the two ends' block counts: [0, mL) from the first, [mR, nB) from the second
 struct BandGeo {
   int P, bw, nB, h, mL, mR, nR;
   __host__ __device__ BandGeo(int N, int D) {
@@ -58,8 +57,12 @@ struct BandGeo {
     bw = 6 * D - 1;
     nB = (P + kBb - 1) / kBb;
     h = (bw + kBb - 1) / kBb;
-    mL = (nB - h + 1) / 2;
-    mR = mL + h;
+    if (nB > h + 1) {
+      mL = (nB - h + 1) / 2;
+      mR = mL + h;
+    } else {
+      mL = mR = nB;
+    }
     nR = nB - mR;
   }
   // first block column of the CTA's factor storage and its step count
@@ -320,7 +323,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBandThreads) k_band
                    "l"(fac + (size_t)c * col + (r - c) * kBb * kBb + 4 * t)
                    : "memory");
   };
-  for (int r = 0; r <= h; ++r)
+  for (int r = 0; r <= min(h, last); ++r)
     for (int t = tid; t < 64 * (r + 1); t += kBandThreads) bring(r, t >> 6, t & 63);
   asm volatile("cp.async.wait_all;" ::: "memory");
   for (int t = tid; t < kBandTri; t += kBandThreads) {  // t -> (r >= c) of a lower triangle
@@ -330,7 +333,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBandThreads) k_band
     tri_c[t] = (unsigned char)(t - r * (r + 1) / 2);
   }
   bd_cluster_sync();  // (also before the peer may raise a flag here)
-  if (warp == 0 && !bd_panel(blocks + bd_slot(0, 0), blocks + bd_slot(1, 0), true, rinv[0], xs, lane)) bad = 1;
+  if (K > 0 && warp == 0 &&
+      !bd_panel(blocks + bd_slot(0, 0), blocks + bd_slot(1, 0), last >= 1, rinv[0], xs, lane))
+    bad = 1;
   __syncthreads();
 
   int km = 0;  // k mod C
@@ -376,7 +381,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBandThreads) k_band
     }
     if (h == 1) asm volatile("cp.async.wait_all;" ::: "memory");  // (then warp 0 reads the new row right away)
     __syncthreads();
-    const bool merge = e == 0 && k == geo.mL - 1;  // the next column is the middle's first
+    const bool merge = e == 0 && geo.nR > 0 && k == geo.mL - 1;  // the next column is the middle's first
     if (warp == 0) {
       if (nr >= 2) bd_update<4, 2>(at(2, 1), at(2, 0), at(1, 0), lane);
       __syncwarp();
@@ -425,7 +430,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBandThreads) k_band
       __syncthreads();
     }
   }
-  if (e == 1) {
+  if (e == 1 && K > 0) {
     // the middle blocks in the first CTA's order and orientation: its block (u, v), element
     // (i, j) is this one's (v', u'), (15 - j, 15 - i)
     for (int t = tid; t < h * (h + 1) / 2 * kBb * kBb; t += kBandThreads) {
@@ -537,14 +542,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBandSolveThreads)
 
   // ---- forward ----
   for (int k = 0; k < kBandStages - 1; ++k) fetch(k, k);
-  for (int s = tid; s < kBb * (h + 1); s += kBandSolveThreads) ring[s] = rhs_at(s);
+  for (int s = tid; s < kBb * (min(h, lastr) + 1); s += kBandSolveThreads) ring[s] = rhs_at(s);
   float rhs_next = d == h + 1 && h + 1 <= lastr ? rhs_at(kBb * (h + 1) + i) : 0.f;  // the block entering at step 0
   bd_cluster_sync();
   float zk = 0.f;
   int km = 0, ks = 0;  // k mod C, k mod kBandStages
   auto wrap = [&](int a) { return a >= C ? a - C : a; };
   for (int k = 0; k < K; ++k) {
-    if (e == 0 && k == geo.mL - 1) {  // the second end's share of the middle
+    if (e == 0 && geo.nR > 0 && k == geo.mL - 1) {  // the second end's share of the middle
       __syncthreads();
       if (tid == 0 && !bd_wait(&peer_done, deadline)) timed_out = 1;
       __syncthreads();
@@ -604,11 +609,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBandSolveThreads)
   if (e == 1 && tid == 0) bd_peer_raise(&peer_done, 0);
 
   // ---- backward ----
-  ks = (K - 1) % kBandStages;
-  km = (K - 1) % C;
+  ks = K > 0 ? (K - 1) % kBandStages : 0;
+  km = K > 0 ? (K - 1) % C : 0;
   for (int q = 0; q < kBandStages - 1; ++q) fetch(K - 1 - q, ks >= q ? ks - q : ks - q + kBandStages);
   float xk = 0.f;  // warp 0: the block after k
-  if (e == 1) {  // the middle's solution from the first CTA
+  if (e == 1 && K > 0) {  // the middle's solution from the first CTA
     if (tid == 0 && !bd_wait(&peer_done, deadline)) timed_out = 1;
     __syncthreads();
     if (!timed_out)
@@ -659,13 +664,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBandSolveThreads)
       xk = both(half_cols(Lk, t));  // x_k = L_kk^-T t
       if (hf == 0) {
         ring[km * kBb + cl] = xk;
-        if (e == 0 && k >= geo.mL) mid[(k - geo.mL) * kBb + cl] = xk;
+        if (e == 0 && geo.nR > 0 && k >= geo.mL) mid[(k - geo.mL) * kBb + cl] = xk;
       }
       keep_z(k, xk);
     } else {
       further(k - 1, mp, stage + sp * stage_len);
     }
-    if (e == 0 && k == geo.mL) {  // the middle is solved: the second end may go on
+    if (e == 0 && geo.nR > 0 && k == geo.mL) {  // the middle is solved: the second end may go on
       __syncthreads();
       if (tid == 0) bd_peer_raise(&peer_done, 1);
     }
@@ -697,11 +702,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBandSolveThreads)
   bd_cluster_sync();  // neither CTA leaves while the other may read its shared memory
 }
 
-// (nB > h + 1: each end has a block column of its own.  The systems too wide for one CTA have at
-// least 19 block rows, so the widest band alone already gives that.)
 bool band_route(int N, int D) {
   const BandGeo g(N, D);
-  return D >= 1 && g.h <= SPGO_BAND_MAX_H && g.nB > g.h + 1 && band_factor_floats(N, D) <= (size_t)g.P * g.P;
+  return D >= 1 && g.h <= SPGO_BAND_MAX_H && band_factor_floats(N, D) <= (size_t)g.P * g.P;
 }
 
 int launch_band_factor(const PlanView &pv, const WorkView &wv, const Params &prm, int b, int N, int D, int sx,
