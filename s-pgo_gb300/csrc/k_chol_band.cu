@@ -60,7 +60,8 @@ struct BandGeo {
     if (nB > h + 1) {
       mL = (nB - h + 1) / 2;
       mR = mL + h;
-    } else {
+    } else {  // one end alone, for a caller with narrow systems: those that come here today have at
+              // least 19 block rows, and h is at most 17
       mL = mR = nB;
     }
     nR = nB - mR;
